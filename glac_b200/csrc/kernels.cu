@@ -523,37 +523,54 @@ template <typename T> __device__ __forceinline__ T su_scalar(double v);
 template <> __device__ __forceinline__ double su_scalar<double>(double v) { return v; }
 template <> __device__ __forceinline__ float su_scalar<float>(double v) { return (float)v; }
 
-GLAC_HD double u_sym16(uint32_t h) { return ((double)h + 0.5) * (1.0 / 65536.0) - 0.5; }
-
-// The same uniform for the FP32 path without a conversion instruction: 2^23 + h
-// read from its bit pattern, minus 2^23, gives h exactly; (h + 1/2) 2^-16 - 1/2
-// = (2h + 1 - 2^16) 2^-17 has at most 17 significant bits, so the FMA is exact
-// and the value equals u_sym16's bit for bit.
+// Proposal uniform (h + 1/2) 2^-16 - 1/2 of a 16-bit word without a conversion
+// instruction: 2^23 + h read from its bit pattern, minus 2^23, gives h exactly;
+// (2h + 1 - 2^16) 2^-17 has at most 17 significant bits, so the FMA is exact.
 __device__ __forceinline__ float u_sym16f(uint32_t h) {
     const float hf = __uint_as_float(0x4B000000u | h) - 8388608.f;
     return __fmaf_rn(hf, 1.f / 65536.f, 0.5f / 65536.f - 0.5f);
 }
+// FP64 the same way: 2^52 + h from its bit pattern (FP64 conversions run on the
+// special-function pipe).
+__device__ __forceinline__ double u32_to_double(uint32_t h) {
+    return __hiloint2double(0x43300000, (int)h) - 4503599627370496.0;
+}
+__device__ __forceinline__ double u_sym16d(uint32_t h) {
+    return __fma_rn(u32_to_double(h), 1.0 / 65536.0, 0.5 / 65536.0 - 0.5);
+}
 template <typename T> __device__ __forceinline__ T proposal_uniform(uint32_t h);
-template <> __device__ __forceinline__ double proposal_uniform<double>(uint32_t h) { return u_sym16(h); }
+template <> __device__ __forceinline__ double proposal_uniform<double>(uint32_t h) { return u_sym16d(h); }
 template <> __device__ __forceinline__ float proposal_uniform<float>(uint32_t h) { return u_sym16f(h); }
 
 // Accept uniform in [0, 1): 53 bits for FP64; for FP32 the 23 high bits of word 6
 // as the mantissa of a float in [1, 2), minus 1 (no conversion instruction).
 template <typename T> __device__ __forceinline__ T accept_uniform(uint32_t w6, uint32_t w7);
-template <> __device__ __forceinline__ double accept_uniform<double>(uint32_t w6, uint32_t w7) { return u_53(w6, w7); }
+template <> __device__ __forceinline__ double accept_uniform<double>(uint32_t w6, uint32_t w7) {
+    // (w6 2^21 + (w7 >> 11)) 2^-53: 53 bits, so the FMA does not round
+    return __fma_rn(u32_to_double(w6), 2097152.0, u32_to_double(w7 >> 11)) * 1.1102230246251565e-16;
+}
 template <> __device__ __forceinline__ float accept_uniform<float>(uint32_t w6, uint32_t) {
     return __uint_as_float(0x3F800000u | (w6 >> 9)) - 1.f;
 }
 
 template <typename T>
-__device__ __forceinline__ void su2_near_unity(T u0, T u1, T u2, T u3, T eps, T sq1me, bool flips, T out[4]) {
-    // x0 = sign(u0) sqrt(1 - eps^2), x = eps u / |u|, normalised
-    // (GLAC/math/matrices/su3matrixgenerator.h:202-243); without flips x0 > 0
-    T x0 = (flips && u0 < T(0)) ? -sq1me : sq1me;
-    T rn = sqrt(u1 * u1 + u2 * u2 + u3 * u3) / eps;
-    T x1 = u1 / rn, x2 = u2 / rn, x3 = u3 / rn;
-    T nrm = sqrt(x0 * x0 + x1 * x1 + x2 * x2 + x3 * x3);
-    out[0] = x0 / nrm; out[1] = x1 / nrm; out[2] = x2 / nrm; out[3] = x3 / nrm;
+__device__ __forceinline__ void su2_near_unity(T u0, T u1, T u2, T u3, T eps, T sq1me, bool flips, T out[4]);
+// x0 = sign(u0) sqrt(1 - eps^2), x = eps u / |u|, normalised
+// (GLAC/math/matrices/su3matrixgenerator.h:202-243); without flips x0 > 0.
+// FP64: |x|^2 = (1 - eps^2) + eps^2 is 1 to a few ulp whatever u is, so the
+// normalisation 1 / sqrt(q) is its first-order term 3/2 - q/2 (the next one is
+// below 1e-30), and u / |u| takes one reciprocal square root: the eight
+// divisions and two square roots of the formula as written had been most of a
+// hit's FP64 operations (four sweeps of 16^3 x 32 on B200: 2.57 ms with them and
+// with converted uniforms, 1.52 ms so).
+template <>
+__device__ __forceinline__ void su2_near_unity<double>(double u0, double u1, double u2, double u3, double eps,
+                                                       double sq1me, bool flips, double out[4]) {
+    const double x0 = (flips && u0 < 0.0) ? -sq1me : sq1me;
+    const double sc = eps * rsqrt(u1 * u1 + u2 * u2 + u3 * u3);
+    const double x1 = u1 * sc, x2 = u2 * sc, x3 = u3 * sc;
+    const double inv = fma(-0.5, x0 * x0 + x1 * x1 + x2 * x2 + x3 * x3, 1.5);
+    out[0] = x0 * inv; out[1] = x1 * inv; out[2] = x2 * inv; out[3] = x3 * inv;
 }
 // FP32: the same construction with reciprocal square roots in place of the
 // square roots and divisions (which load the special-function pipe).

@@ -305,12 +305,4 @@ GLAC_HD U4 philox4x32_10(U4 c, uint32_t k0, uint32_t k1) {
     return c;
 }
 
-// uniform in (-1/2, 1/2), never 0
-GLAC_HD double u_sym(uint32_t w) { return ((double)w + 0.5) * 2.3283064365386963e-10 - 0.5; }
-GLAC_HD float u_symf(uint32_t w) { return ((float)(w >> 8) + 0.5f) * 5.9604644775390625e-8f - 0.5f; }
-// uniform in [0,1) with 53 bits
-GLAC_HD double u_53(uint32_t hi, uint32_t lo) {
-    return (double)(((uint64_t)hi << 21) | (lo >> 11)) * 1.1102230246251565e-16;
-}
-
 }  // namespace glac
