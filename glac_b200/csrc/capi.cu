@@ -278,7 +278,7 @@ glac_status glac_create(const glac_desc *desc, glac_ctx **out) {
     c->plan = make_obs_plan(c->g);
     // the faster fused-measurement kernel per precision on B200 at 32^3 x 64:
     // FP32 with the 128-register cap (2.50 vs 2.61 ms per measured flow step),
-    // FP64 uncapped (6.33 vs 6.77 ms)
+    // FP64 at three blocks per SM (1.51 vs 1.65 ms at 24^3 x 48)
     c->fused_measure = d.precision == GLAC_FP32 ? 2 : 1;
     try {
         ck(cudaSetDevice(d.device), "cudaSetDevice");

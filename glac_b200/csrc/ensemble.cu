@@ -218,9 +218,8 @@ template <typename T> void flow_t(glac_ensemble *E, int n, bool measure) {
     for (int step = 0; step < n; step++) {
         for (int stage = 0; stage < 3; stage++) {
             if (stage == 0 && fused) {
-                // FP32: the 128-register kernel, FP64: the compiler's own allocation
                 launch_ens_flow_stage0_meas<T>(slots_of<T>(E), E->start[ENS_FLOW0], E->nblk[ENS_FLOW0], E->M, cur,
-                                               3 - cur, alpha[0], sizeof(T) == 4 ? 128 : 0, E->stream);
+                                               3 - cur, alpha[0], E->stream);
                 launch_ens_obs_combine<T>(slots_of<T>(E), E->start[ENS_OBS], E->nblk[ENS_OBS], E->M, step,
                                           E->stream);
                 E->launches += 3;

@@ -54,6 +54,13 @@ __device__ __forceinline__ int tiled_chunk(const Geom &g, int j) {
     return k + K * (z + g.N[2] * t);
 }
 
+// Force of a link from its staple sum.  FP64 forms only the part of U A that
+// enters; in FP32 at 80 registers the full product was the faster one.
+template <typename T> __device__ __forceinline__ AH8<T> flow_force(const M3<T> &U, const M3<T> &A) {
+    if constexpr (sizeof(T) == 4) return project_ah(mul(U, A));
+    else return project_ah_mul(U, A);
+}
+
 template <typename T, int KIND, int STAGE, int SHAPE>
 __device__ __forceinline__ void flow_stage_body(const Geom &g, const LinkField<T> &in, const LinkField<T> &out,
                                                 const ForceField<T> &zf, T alpha, T beta, int bx) {
@@ -66,7 +73,7 @@ __device__ __forceinline__ void flow_stage_body(const Geom &g, const LinkField<T
     const Site n = site_from_ps(g, p, s);
     M3<T> A = staple<T, false, true>(in, g, n, p, mu);
     const M3<T> U = in.load(mu, p, s);
-    const AH8<T> Z = project_ah(mul(U, A));
+    const AH8<T> Z = flow_force(U, A);
     AH8<T> M;
     if (STAGE == 0) {
         M = ah_scale(alpha, Z);
@@ -236,8 +243,12 @@ GLAC_FLOW_KERNEL(k_flow_stage_r96, __maxnreg__(96))
 // Launch-bound variants (minimum resident blocks of 128 threads per SM, i.e.
 // the register cap) that the autotuner chooses among; variant 0 is the default.
 // Register caps per variant ([fp64, fp32]; 0 = no cap, -1 = unused slot); the
-// flow family also varies the site-block shape.
-const int kFlowRegs[2][kMaxVariants] = {{0, 128, 0, 128}, {0, 80, 0, 96}};
+// flow family also varies the site-block shape.  The flow stage waits on its
+// neighbour links (L2 hits), so resident warps count for more than registers:
+// its default caps give 16 (FP64) and 24 (FP32) warps per SM.  Stage 2 on B200,
+// capped / uncapped: FP64 24^3 x 48 427 / 528 us, 16^3 x 32 97 / 114; FP32
+// 32^3 x 64 662 / 700, 16^3 x 32 51 / 53.
+const int kFlowRegs[2][kMaxVariants] = {{128, 0, 0, 128}, {80, 0, 0, 96}};
 const int kFlowShape[2][kMaxVariants] = {{0, 0, 1, 2}, {0, 0, 3, 0}};
 const int kMetroRegs[2][kMaxVariants] = {{0, 128, -1, -1}, {0, 96, 80, 128}};
 const int kObsRegs[2][kMaxVariants] = {{0, 128, -1, -1}, {0, 128, 168, -1}};
@@ -380,6 +391,13 @@ template <typename T> __device__ __forceinline__ AH8<T> ah_neg_if(const AH8<T> &
     return neg ? ah_scale(T(-1), F) : F;
 }
 
+// P(A B), negated where neg: twice project_ah of the product, with its sign turned
+// (FP64; FP32 forms the product, as flow_force).
+template <typename T> __device__ __forceinline__ AH8<T> clover_part(const M3<T> &A, const M3<T> &B, bool neg) {
+    if constexpr (sizeof(T) == 4) return ah_neg_if(proj_ah8(mul(A, B)), neg);
+    else return ah_scale(neg ? T(2) : T(-2), project_ah_mul(A, B));
+}
+
 template <typename T, int KIND>
 __device__ __forceinline__ void flow_stage0_meas_body(const Geom &g, const LinkField<T> &in, const LinkField<T> &out,
                                                       const ForceField<T> &zf, const CloverParts<T> &cp, T alpha,
@@ -389,7 +407,7 @@ __device__ __forceinline__ void flow_stage0_meas_body(const Geom &g, const LinkF
     if (s >= g.Vh) return;
     const int mu = plane >> 1, p = plane & 1, q = p ^ 1;
     const Site n = site_from_ps(g, p, s);
-    const int f_mu = sizeof(T) == 4 ? step_offset(g, n, mu, +1) : step_offset_indexed(g, n, mu, +1);
+    const int f_mu = step_offset(g, n, mu, +1);
     const int s_mu = (n.lex + f_mu) >> 1;
     M3<T> A;
     set_zero(A);
@@ -397,17 +415,9 @@ __device__ __forceinline__ void flow_stage0_meas_body(const Geom &g, const LinkF
 #pragma unroll 1
     for (int nu = 0; nu < 4; nu++) {
         if (nu == mu) continue;
-        int s_nup, s_num, s_diag;
-        if constexpr (sizeof(T) == 4) {
-            const int b_nu = step_offset(g, n, nu, -1);
-            s_nup = (n.lex + step_offset(g, n, nu, +1)) >> 1;
-            s_num = (n.lex + b_nu) >> 1;
-            s_diag = (n.lex + f_mu + b_nu) >> 1;
-        } else {
-            s_nup = lex_step(g, n, nu, +1) >> 1;
-            s_num = lex_step(g, n, nu, -1) >> 1;
-            s_diag = lex_step2(g, n, mu, +1, nu, -1) >> 1;
-        }
+        const int b_nu = step_offset(g, n, nu, -1);
+        const int s_nup = (n.lex + step_offset(g, n, nu, +1)) >> 1, s_num = (n.lex + b_nu) >> 1,
+                  s_diag = (n.lex + f_mu + b_nu) >> 1;
         if (!meas_takes(mu, nu)) {
             {
                 M3<T> t = flow_nd(in.load(nu, q, s_mu), in.load(mu, q, s_nup));
@@ -437,13 +447,13 @@ __device__ __forceinline__ void flow_stage0_meas_body(const Geom &g, const LinkF
         const bool neg = nu < mu;  // F_numu = -F_munu
         const int pl = neg ? plane_of(nu, mu) : plane_of(mu, nu);
         asm volatile("" ::: "memory");
-        cp.ah.store(2 * pl, p, s, ah_neg_if(proj_ah8(mul(in.load(mu, p, s), W)), neg));
+        cp.ah.store(2 * pl, p, s, clover_part(in.load(mu, p, s), W, neg));
         asm volatile("" ::: "memory");
-        cp.ah.store(2 * pl + 1, q, s_mu, ah_neg_if(proj_ah8(mul(W, in.load(mu, p, s))), neg));
+        cp.ah.store(2 * pl + 1, q, s_mu, clover_part(W, in.load(mu, p, s), neg));
     }
     cp.plaq[(mu * 2 + p) * g.Vh + s] = plaq;
     const M3<T> U = in.load(mu, p, s);
-    const AH8<T> Z = project_ah(mul(U, A));
+    const AH8<T> Z = flow_force(U, A);
     zf.store(mu, p, s, Z);
     const AH8<T> M = ah_scale(alpha, Z);
     if (KIND == EXP_MORNINGSTAR) out.store(mu, p, s, mul_plus_right(expm_morningstar<T, true>(M), U));
@@ -457,6 +467,9 @@ __device__ __forceinline__ void flow_stage0_meas_body(const Geom &g, const LinkF
         flow_stage0_meas_body<T, KIND>(g, in, out, zf, cp, alpha, blockIdx.x);                           \
     }
 GLAC_FLOW_MEAS_KERNEL(k_flow_stage0_meas, __launch_bounds__(128))
+// FP64's form 1: three blocks per SM (168 registers, 40 B spill), 598 us at
+// 24^3 x 48 on B200; at the compiler's 252 registers and two blocks 633, at 128 735.
+GLAC_FLOW_MEAS_KERNEL(k_flow_stage0_meas_b3, __launch_bounds__(128, 3))
 GLAC_FLOW_MEAS_KERNEL(k_flow_stage0_meas_r128, __maxnreg__(128))
 GLAC_FLOW_MEAS_KERNEL(k_flow_stage0_meas_r96, __maxnreg__(96))
 #undef GLAC_FLOW_MEAS_KERNEL
@@ -467,6 +480,18 @@ __global__ void __launch_bounds__(kSiteBlock) k_flow_stage0_meas_site(Geom g, Li
                                                                       ForceField<T> zf, CloverParts<T> cp, T alpha) {
     __shared__ T slots[4 * 18 * kSiteBlock];
     flow_stage_site_body<T, KIND, 0, true>(g, in, out, zf, alpha, T(0), blockIdx.x, slots, &cp);
+}
+
+template <typename T, int KIND>
+static void meas_dispatch(int regs, dim3 grid, cudaStream_t st, const Geom &g, const LinkField<T> &in,
+                          const LinkField<T> &out, const ForceField<T> &zf, const CloverParts<T> &cp, T a) {
+    if (regs == 128) {
+        k_flow_stage0_meas_r128<T, KIND><<<grid, 128, 0, st>>>(g, in, out, zf, cp, a);
+        return;
+    }
+    if constexpr (sizeof(T) == 8) k_flow_stage0_meas_b3<T, KIND><<<grid, 128, 0, st>>>(g, in, out, zf, cp, a);
+    else if (regs == 96) k_flow_stage0_meas_r96<T, KIND><<<grid, 128, 0, st>>>(g, in, out, zf, cp, a);
+    else k_flow_stage0_meas<T, KIND><<<grid, 128, 0, st>>>(g, in, out, zf, cp, a);
 }
 
 template <typename T>
@@ -486,15 +511,12 @@ void launch_flow_stage0_meas(const Geom &g, const LinkField<T> &in, const LinkFi
             }
         }
     }
-#define GLAC_MEAS_CASE(K)                                                                                 \
-    if (kind == K) {                                                                                      \
-        if (regs == 128) k_flow_stage0_meas_r128<T, K><<<grid, 128, 0, st>>>(g, in, out, zf, cp, a);        \
-        else if (regs == 96) k_flow_stage0_meas_r96<T, K><<<grid, 128, 0, st>>>(g, in, out, zf, cp, a);     \
-        else k_flow_stage0_meas<T, K><<<grid, 128, 0, st>>>(g, in, out, zf, cp, a);                       \
-        return;                                                                                           \
+    switch (kind) {
+    case 0: meas_dispatch<T, 0>(regs, grid, st, g, in, out, zf, cp, a); return;
+    case 1: meas_dispatch<T, 1>(regs, grid, st, g, in, out, zf, cp, a); return;
+    case 2: meas_dispatch<T, 2>(regs, grid, st, g, in, out, zf, cp, a); return;
+    case 3: meas_dispatch<T, 3>(regs, grid, st, g, in, out, zf, cp, a); return;
     }
-    GLAC_MEAS_CASE(0) GLAC_MEAS_CASE(1) GLAC_MEAS_CASE(2) GLAC_MEAS_CASE(3)
-#undef GLAC_MEAS_CASE
     throw std::invalid_argument("bad exp kind");
 }
 template void launch_flow_stage0_meas<double>(const Geom &, const LinkField<double> &, const LinkField<double> &,
@@ -1139,9 +1161,9 @@ __global__ void __launch_bounds__(256) k_obs_combine(Geom g, CloverParts<T> cp, 
 // slice and its partial sums sit where the observable plan's 128-site blocks
 // put them (obs_combine_in_stage1).  Launch bounds: six blocks of 128 per SM
 // in FP32 (80 registers, 12 B spill; 3 % faster than five blocks at 96 on
-// B200), three in FP64.
+// B200), four in FP64 (128 registers: 483 us at 24^3 x 48 on B200, 489 at three).
 template <typename T, int KIND>
-__global__ void __launch_bounds__(128, sizeof(T) == 4 ? 6 : 3) k_flow_stage1_combine(Geom g, LinkField<T> in, LinkField<T> out,
+__global__ void __launch_bounds__(128, sizeof(T) == 4 ? 6 : 4) k_flow_stage1_combine(Geom g, LinkField<T> in, LinkField<T> out,
                                                              ForceField<T> zf, T alpha, T beta, CloverParts<T> cp,
                                                              double *partial) {
     flow_stage_body<T, KIND, 1, 0>(g, in, out, zf, alpha, beta, blockIdx.x);
@@ -1902,15 +1924,17 @@ void launch_ens_observables(const LatSlot<T> *slots, const int *start, int nbloc
         flow_stage0_meas_body<T, EXP_MORNINGSTAR>(S.g, S.f[src], S.f[dst], S.z, S.cp, alpha,                \
                                                   blockIdx.x - __ldg(start + i));                          \
     }
-GLAC_ENS_MEAS_KERNEL(kb_flow_stage0_meas, __launch_bounds__(128))
+GLAC_ENS_MEAS_KERNEL(kb_flow_stage0_meas_b3, __launch_bounds__(128, 3))
 GLAC_ENS_MEAS_KERNEL(kb_flow_stage0_meas_r128, __maxnreg__(128))
 #undef GLAC_ENS_MEAS_KERNEL
 
 template <typename T>
 void launch_ens_flow_stage0_meas(const LatSlot<T> *slots, const int *start, int nblocks, int M, int src, int dst,
-                                 double alpha, int regs, cudaStream_t st) {
-    if (regs == 128) kb_flow_stage0_meas_r128<T><<<nblocks, 128, 0, st>>>(slots, start, M, src, dst, (T)alpha);
-    else kb_flow_stage0_meas<T><<<nblocks, 128, 0, st>>>(slots, start, M, src, dst, (T)alpha);
+                                 double alpha, cudaStream_t st) {
+    // the forms of the single-lattice launch: FP32 at 128 registers, FP64 at three blocks per SM
+    if constexpr (sizeof(T) == 4)
+        kb_flow_stage0_meas_r128<T><<<nblocks, 128, 0, st>>>(slots, start, M, src, dst, (T)alpha);
+    else kb_flow_stage0_meas_b3<T><<<nblocks, 128, 0, st>>>(slots, start, M, src, dst, (T)alpha);
 }
 
 template <typename T>
@@ -2111,7 +2135,7 @@ void launch_advance(uint32_t *counter, uint32_t by, cudaStream_t st) { k_advance
     template void launch_ens_observables<T>(const LatSlot<T> *, const int *, int, int, int, int, int,         \
                                             cudaStream_t);                                                    \
     template void launch_ens_flow_stage0_meas<T>(const LatSlot<T> *, const int *, int, int, int, int, double, \
-                                                 int, cudaStream_t);                                          \
+                                                 cudaStream_t);                                          \
     template void launch_ens_obs_combine<T>(const LatSlot<T> *, const int *, int, int, int, cudaStream_t);
 GLAC_ENS_INST(double)
 GLAC_ENS_INST(float)

@@ -38,15 +38,17 @@ __device__ __forceinline__ M3<T> staple(const LinkField<T> &L, const Geom &g, co
     M3<T> A;
     set_zero(A);
     const int q = p ^ 1;
-    // Neighbour indices: select chains in FP32 (pick4), indexed arrays in FP64;
-    // each form is the faster one for its precision.
-    const int f_mu = sizeof(T) == 4 ? step_offset(g, n, mu, +1) : step_offset_indexed(g, n, mu, +1);
+    // Neighbour indices: select chains (pick4) in FP32 and in the flow stage,
+    // indexed arrays in the FP64 Metropolis kernel; each form is the faster one
+    // there (FP64 flow stage at 128 registers, 24^3 x 48 on B200: 423 against 449 us).
+    constexpr bool sel = sizeof(T) == 4 || RECON;
+    const int f_mu = sel ? step_offset(g, n, mu, +1) : step_offset_indexed(g, n, mu, +1);
     const int s_mu = (n.lex + f_mu) >> 1;
 #pragma unroll(UNROLL ? 4 : 1)
     for (int nu = 0; nu < 4; nu++) {
         if (nu == mu) continue;
         int s_nup, s_num, s_diag;
-        if constexpr (sizeof(T) == 4) {
+        if constexpr (sel) {
             const int b_nu = step_offset(g, n, nu, -1);
             s_nup = (n.lex + step_offset(g, n, nu, +1)) >> 1;
             s_num = (n.lex + b_nu) >> 1;
@@ -209,7 +211,7 @@ void launch_ens_observables(const LatSlot<T> *slots, const int *start, int nbloc
 // measurement row `meas` (block table of the observable phase).
 template <typename T>
 void launch_ens_flow_stage0_meas(const LatSlot<T> *slots, const int *start, int nblocks, int M, int src, int dst,
-                                 double alpha, int regs, cudaStream_t st);
+                                 double alpha, cudaStream_t st);
 template <typename T>
 void launch_ens_obs_combine(const LatSlot<T> *slots, const int *start, int nblocks, int M, int meas,
                             cudaStream_t st);

@@ -362,6 +362,39 @@ template <> GLAC_HD AH8<double> project_ah<double>(const M3<double> &X) {
     return Z;
 }
 
+// project_ah(A B) from 90 multiply-adds instead of 108: only X_ji^* - X_ij and the
+// imaginary diagonal of X = A B enter, and the differences ride in the
+// accumulators.
+template <typename R> GLAC_HD AH8<R> project_ah_mul(const M3<R> &A, const M3<R> &B) {
+    R m[3];
+#pragma unroll
+    for (int i = 0; i < 3; i++) {
+        m[i] = rzero<R>();
+#pragma unroll
+        for (int k = 0; k < 3; k++) {
+            m[i] = fmaR(A(i, k).re, B(k, i).im, m[i]);
+            m[i] = fmaR(A(i, k).im, B(k, i).re, m[i]);
+        }
+    }
+    const R tr = (m[0] + m[1] + m[2]) / R(3.f);
+    auto off = [&](int i, int j) {
+        Cx<R> s = cx(rzero<R>(), rzero<R>());
+#pragma unroll
+        for (int k = 0; k < 3; k++) {
+            s = cmac_cc(s, A(j, k), B(k, i));
+            s = cmac(s, -A(i, k), B(k, j));
+        }
+        return cx(s.re * R(0.5f), s.im * R(0.5f));
+    };
+    AH8<R> Z;
+    Z.a = tr - m[0];
+    Z.d = tr - m[1];
+    Z.b = off(0, 1);
+    Z.c = off(0, 2);
+    Z.e = off(1, 2);
+    return Z;
+}
+
 template <typename R> GLAC_HD M3<R> ah_to_m3(const AH8<R> &Z) {
     M3<R> M;
     R z = rzero<R>();
