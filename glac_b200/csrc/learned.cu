@@ -336,8 +336,10 @@ void launch_mlp_forward_tc(const float *params, const float *features, long long
 // J_i(eps) linear between grid points; returns J and its slope.
 __device__ __forceinline__ float esj_interp(const float *__restrict__ J, const float *__restrict__ grid, int n_eps,
                                             float eps, float &slope) {
+    // grid points 1 .. n_eps - 2 at or below eps (the grid increases); the loads
+    // do not wait for one another as a search's would
     int k = 0;
-    while (k < n_eps - 2 && grid[k + 1] <= eps) k++;
+    for (int j = 1; j < n_eps - 1; j++) k += grid[j] <= eps ? 1 : 0;
     const float e0 = grid[k], e1 = grid[k + 1];
     const float j0 = __ldg(J + k), j1 = __ldg(J + k + 1);
     slope = (j1 - j0) / (e1 - e0);
@@ -348,27 +350,67 @@ __device__ __forceinline__ float esj_interp(const float *__restrict__ J, const f
 // caller picks the word for rows g / g+8.
 __device__ __forceinline__ float bf_el(uint32_t w, int c) { return c == 0 ? bf16_lo(w) : bf16_hi(w); }
 
-__global__ void __launch_bounds__(128) k_mlp_grad(const float *__restrict__ P, const uint32_t *__restrict__ pack,
+__device__ __forceinline__ void prefetch_l1(const void *p) { asm volatile("prefetch.global.L1 [%0];" ::"l"(p)); }
+// Packed fragments by a coherent load: the step before may write them while this kernel starts.
+__device__ __forceinline__ uint2 ld_pack(const uint32_t *p) {
+    uint2 v;
+    asm volatile("ld.global.v2.u32 {%0, %1}, [%2];" : "=r"(v.x), "=r"(v.y) : "l"(p) : "memory");
+    return v;
+}
+
+// With one tile to a warp (batches up to 18,944 rows) the pass is a chain of
+// load latencies, so what does not depend on the last step's parameters (rows,
+// grid) is fetched before the wait for it, and the fragments together after it.
+__global__ void __launch_bounds__(128) k_mlp_grad(const float *P, const uint32_t *pack,
                                                   const float *__restrict__ feat, const float *__restrict__ esj,
                                                   long long n, int n_eps, const float *__restrict__ eps_grid,
                                                   float eps_min, float eps_max, float *__restrict__ partial) {
     __shared__ float red[kGradWarps][kGradSlots];
     __shared__ float grid_s[64];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, t = lane & 3;
-    for (int k = threadIdx.x; k < n_eps; k += blockDim.x) grid_s[k] = eps_grid[k];
-    __syncthreads();
     const long long ntiles = (n + 15) / 16;
     const long long nw = (long long)gridDim.x * kGradWarps;
+    // rows of a tile: features into registers, the lines of J on their way to L1
+    auto fetch = [&](long long tile, float2 &x0, float2 &x1) {
+        const long long r0 = tile * 16 + g, r1 = r0 + 8;
+        x0 = x1 = make_float2(0.f, 0.f);
+        if (r0 < n) {
+            x0 = __ldg(reinterpret_cast<const float2 *>(feat + r0 * 8 + 2 * t));
+            prefetch_l1(esj + r0 * n_eps + min(32 * t, n_eps - 1));
+        }
+        if (r1 < n) {
+            x1 = __ldg(reinterpret_cast<const float2 *>(feat + r1 * 8 + 2 * t));
+            prefetch_l1(esj + r1 * n_eps + min(32 * t, n_eps - 1));
+        }
+    };
+    // none of this is written by the step before, so it may run beside its end
+    for (int k = threadIdx.x; k < n_eps; k += blockDim.x) grid_s[k] = eps_grid[k];
+    float2 x0, x1;
+    fetch((long long)blockIdx.x * kGradWarps + warp, x0, x1);
+    cudaTriggerProgrammaticLaunchCompletion();
+    cudaGridDependencySynchronize();
+    __syncthreads();
     const float inv_n = 1.f / (float)n, span = eps_max - eps_min;
     const uint32_t one = t == 0 ? pack_bf16(1.f, 0.f) : 0u;
-    const float *b2 = reinterpret_cast<const float *>(pack + kPackB2);
+    // the network's fragments once per warp
     const float b3 = reinterpret_cast<const float *>(pack + kPackB3)[0];
+    uint2 fW1[4], fW2[2][4], fW3[2], fW2T[2][4];
+    float2 b2[4];
     float w3[4][2];
 #pragma unroll
     for (int nt = 0; nt < 4; nt++) {
+        fW1[nt] = ld_pack(pack + kPackW1 + (nt * 32 + lane) * 2);
+        b2[nt] = *reinterpret_cast<const float2 *>(pack + kPackB2 + 8 * nt + 2 * t);
         w3[nt][0] = round_bf16(P[kMlpW3 + 8 * nt + 2 * t]);
         w3[nt][1] = round_bf16(P[kMlpW3 + 8 * nt + 2 * t + 1]);
+#pragma unroll
+        for (int ks = 0; ks < 2; ks++) {
+            fW2[ks][nt] = ld_pack(pack + kPackW2 + ((ks * 4 + nt) * 32 + lane) * 2);
+            fW2T[ks][nt] = ld_pack(pack + kPackW2T + ((ks * 4 + nt) * 32 + lane) * 2);
+        }
     }
+#pragma unroll
+    for (int ks = 0; ks < 2; ks++) fW3[ks] = ld_pack(pack + kPackW3 + (ks * 32 + lane) * 2);
     float gW1[4][4], gW2[2][4][4], gb1[4][2], gb2[4][2], gW3[4][2], gb3 = 0.f, loss = 0.f;
 #pragma unroll
     for (int nt = 0; nt < 4; nt++) {
@@ -381,9 +423,8 @@ __global__ void __launch_bounds__(128) k_mlp_grad(const float *__restrict__ P, c
     for (long long tile = (long long)blockIdx.x * kGradWarps + warp; tile < ntiles; tile += nw) {
         const long long r0 = tile * 16 + g, r1 = r0 + 8;
         const bool v0 = r0 < n, v1 = r1 < n;
-        const float2 x0 = v0 ? __ldg(reinterpret_cast<const float2 *>(feat + r0 * 8 + 2 * t)) : make_float2(0.f, 0.f);
-        const float2 x1 = v1 ? __ldg(reinterpret_cast<const float2 *>(feat + r1 * 8 + 2 * t)) : make_float2(0.f, 0.f);
         const uint32_t a0 = pack_bf16(x0.x, x0.y), a1 = pack_bf16(x1.x, x1.y);
+        if (tile + nw < ntiles) fetch(tile + nw, x0, x1);
 
         // forward; h1/h2 hold the BF16 activations in the A-operand order, which
         // is also the C layout: [nt >> 1][2 (nt & 1) + half], half 0 = row g, 1 = row g+8
@@ -391,28 +432,23 @@ __global__ void __launch_bounds__(128) k_mlp_grad(const float *__restrict__ P, c
 #pragma unroll
         for (int nt = 0; nt < 4; nt++) {
             float c[4] = {0.f, 0.f, 0.f, 0.f};
-            const uint2 b = ld_frag(pack + kPackW1 + (nt * 32 + lane) * 2);
-            mma_bf16(c, a0, a1, one, one, b.x, b.y);
+            mma_bf16(c, a0, a1, one, one, fW1[nt].x, fW1[nt].y);
             h1[nt >> 1][2 * (nt & 1)] = pack_bf16(leaky(c[0]), leaky(c[1]));
             h1[nt >> 1][2 * (nt & 1) + 1] = pack_bf16(leaky(c[2]), leaky(c[3]));
         }
 #pragma unroll
         for (int nt = 0; nt < 4; nt++) {
-            float c[4] = {b2[8 * nt + 2 * t], b2[8 * nt + 2 * t + 1], b2[8 * nt + 2 * t], b2[8 * nt + 2 * t + 1]};
+            float c[4] = {b2[nt].x, b2[nt].y, b2[nt].x, b2[nt].y};
 #pragma unroll
-            for (int ks = 0; ks < 2; ks++) {
-                const uint2 b = ld_frag(pack + kPackW2 + ((ks * 4 + nt) * 32 + lane) * 2);
-                mma_bf16(c, h1[ks][0], h1[ks][1], h1[ks][2], h1[ks][3], b.x, b.y);
-            }
+            for (int ks = 0; ks < 2; ks++)
+                mma_bf16(c, h1[ks][0], h1[ks][1], h1[ks][2], h1[ks][3], fW2[ks][nt].x, fW2[ks][nt].y);
             h2[nt >> 1][2 * (nt & 1)] = pack_bf16(leaky(c[0]), leaky(c[1]));
             h2[nt >> 1][2 * (nt & 1) + 1] = pack_bf16(leaky(c[2]), leaky(c[3]));
         }
         float c3[4] = {b3, b3, b3, b3};
 #pragma unroll
-        for (int ks = 0; ks < 2; ks++) {
-            const uint2 b = ld_frag(pack + kPackW3 + (ks * 32 + lane) * 2);
-            mma_bf16(c3, h2[ks][0], h2[ks][1], h2[ks][2], h2[ks][3], b.x, b.y);
-        }
+        for (int ks = 0; ks < 2; ks++)
+            mma_bf16(c3, h2[ks][0], h2[ks][1], h2[ks][2], h2[ks][3], fW3[ks].x, fW3[ks].y);
         const float zq[2] = {__shfl_sync(0xffffffffu, c3[0], lane & ~3), __shfl_sync(0xffffffffu, c3[2], lane & ~3)};
 
         // dL/dz of rows g and g+8 (every lane of the quad computes both)
@@ -469,10 +505,8 @@ __global__ void __launch_bounds__(128) k_mlp_grad(const float *__restrict__ P, c
         for (int nt = 0; nt < 4; nt++) {
             float c[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
-            for (int ks = 0; ks < 2; ks++) {
-                const uint2 b = ld_frag(pack + kPackW2T + ((ks * 4 + nt) * 32 + lane) * 2);
-                mma_bf16(c, d2[ks][0], d2[ks][1], d2[ks][2], d2[ks][3], b.x, b.y);
-            }
+            for (int ks = 0; ks < 2; ks++)
+                mma_bf16(c, d2[ks][0], d2[ks][1], d2[ks][2], d2[ks][3], fW2T[ks][nt].x, fW2T[ks][nt].y);
             const uint32_t hg = h1[nt >> 1][2 * (nt & 1)], hg8 = h1[nt >> 1][2 * (nt & 1) + 1];
             const float e0 = c[0] * leaky_slope(bf16_lo(hg)), e1 = c[1] * leaky_slope(bf16_hi(hg));
             const float e2 = c[2] * leaky_slope(bf16_lo(hg8)), e3 = c[3] * leaky_slope(bf16_hi(hg8));
@@ -537,14 +571,63 @@ __global__ void __launch_bounds__(128) k_mlp_grad(const float *__restrict__ P, c
         partial[(long long)blockIdx.x * kGradSlots + k] = ((red[0][k] + red[1][k]) + red[2][k]) + red[3][k];
 }
 
-__global__ void k_mlp_reduce(const float *__restrict__ partial, int nblocks, float *__restrict__ grad,
-                             float *__restrict__ loss) {
-    const int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= kGradSlots) return;
+// Parameter k's places in the packed fragments (k_mlp_pack's words by parameter).
+__device__ __forceinline__ void pack_param(uint32_t *pack, int k, float v) {
+    __nv_bfloat16 *half = reinterpret_cast<__nv_bfloat16 *>(pack);
+    // element (row, col) of a B operand whose 16 x 8 tiles have `nts` tiles a K step
+    auto put = [&](int base, int nts, int row, int col) {
+        const int ks = row >> 4, r = (row >> 3) & 1, t = (row & 7) >> 1, lane = 4 * (col & 7) + t;
+        half[2 * (base + ((ks * nts + (col >> 3)) * 32 + lane) * 2 + r) + (row & 1)] = __float2bfloat16_rn(v);
+    };
+    if (k < kMlpB1) put(kPackW1, 4, k >> 5, k & 31);
+    else if (k < kMlpW2) put(kPackW1, 4, 8, k - kMlpB1);
+    else if (k < kMlpB2) {
+        const int i = (k - kMlpW2) >> 5, j = (k - kMlpW2) & 31;
+        put(kPackW2, 4, i, j);
+        put(kPackW2T, 4, j, i);
+    } else if (k < kMlpW3) pack[kPackB2 + (k - kMlpB2)] = __float_as_uint(v);
+    else if (k < kMlpB3) put(kPackW3, 1, k - kMlpW3, 0);
+    else pack[kPackB3] = __float_as_uint(v);
+}
+
+// Sum of the block partials in block order, 32 slots to a block: all threads
+// bring the partials in together, one warp adds them.  STEP: the Adam update
+// (Kingma & Ba, arXiv:1412.6980, Algorithm 1; beta1 0.9, beta2 0.999, eps 1e-8)
+// and the parameter's packed fragments follow at once, where separate launches
+// for the sum (a serial chain of L2 loads), Adam and packing took 16 of the
+// 22.8 us of a step of 8192 rows on B200.
+constexpr int kStepThreads = 256;
+template <bool STEP>
+__global__ void __launch_bounds__(kStepThreads) k_mlp_step(const float *partial, int nblocks, float *grad, float *loss,
+                                                           float *p, float *m, float *v, uint32_t *pack, float lr,
+                                                           float c1, float c2) {
+    __shared__ float rows[kGradMaxBlocks][32];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, k = blockIdx.x * 32 + lane;
+    cudaTriggerProgrammaticLaunchCompletion();
+    cudaGridDependencySynchronize();
+#pragma unroll 8
+    for (int b = warp; b < nblocks; b += kStepThreads / 32)
+        rows[b][lane] = k < kGradSlots ? partial[(long long)b * kGradSlots + k] : 0.f;
+    __syncthreads();
+    if (warp != 0 || k >= kGradSlots) return;
     float s = 0.f;
-    for (int b = 0; b < nblocks; b++) s += partial[(long long)b * kGradSlots + k];
-    if (k < kMlpParams) grad[k] = s;
-    else loss[0] = s;
+#pragma unroll 8
+    for (int b = 0; b < nblocks; b++) s += rows[b][lane];
+    if (k == kMlpParams) {
+        loss[0] = s;
+        return;
+    }
+    if (!STEP) {
+        grad[k] = s;
+        return;
+    }
+    const float mk = 0.9f * m[k] + 0.1f * s;
+    const float vk = 0.999f * v[k] + 0.001f * s * s;
+    m[k] = mk;
+    v[k] = vk;
+    const float pk = p[k] - lr * (mk / c1) / (sqrtf(vk / c2) + 1e-8f);
+    p[k] = pk;
+    pack_param(pack, k, pk);
 }
 
 static int grad_blocks(long long n) {
@@ -556,30 +639,42 @@ static int grad_blocks(long long n) {
 
 size_t mlp_grad_scratch(long long n) { return (size_t)grad_blocks(n) * kGradSlots; }
 
+// Launch that may start while the kernel before it drains (both wait for its
+// end, by cudaGridDependencySynchronize, before they touch what it writes).
+template <typename... Params, typename... Args>
+static void launch_chained(void (*kernel)(Params...), int grid, int threads, cudaStream_t st, Args... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)grid);
+    cfg.blockDim = dim3((unsigned)threads);
+    cfg.stream = st;
+    cudaLaunchAttribute at = {};
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    cudaLaunchKernelEx(&cfg, kernel, static_cast<Params>(args)...);
+}
+
 void launch_mlp_grad(const float *params, const uint32_t *pack, const float *features, const float *esj, long long n,
                      int n_eps, const float *eps_grid_dev, float eps_min, float eps_max, float *partial, float *grad,
                      float *loss, cudaStream_t st) {
     const int nb = grad_blocks(n);
-    k_mlp_grad<<<nb, 128, 0, st>>>(params, pack, features, esj, n, n_eps, eps_grid_dev, eps_min, eps_max, partial);
-    k_mlp_reduce<<<(kGradSlots + 255) / 256, 256, 0, st>>>(partial, nb, grad, loss);
+    launch_chained(k_mlp_grad, nb, 128, st, params, pack, features, esj, n, n_eps, eps_grid_dev, eps_min, eps_max,
+                   partial);
+    launch_chained(k_mlp_step<false>, (kGradSlots + 31) / 32, kStepThreads, st, partial, nb, grad, loss,
+                   static_cast<float *>(nullptr), static_cast<float *>(nullptr), static_cast<float *>(nullptr),
+                   static_cast<uint32_t *>(nullptr), 0.f, 1.f, 1.f);
 }
 
-// Adam (Kingma & Ba, arXiv:1412.6980, Algorithm 1), beta1 0.9, beta2 0.999, eps 1e-8.
-__global__ void k_adam(float *__restrict__ p, float *__restrict__ m, float *__restrict__ v,
-                       const float *__restrict__ grad, float lr, float c1, float c2) {
-    const int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= kMlpParams) return;
-    const float gk = grad[k];
-    const float mk = 0.9f * m[k] + 0.1f * gk;
-    const float vk = 0.999f * v[k] + 0.001f * gk * gk;
-    m[k] = mk;
-    v[k] = vk;
-    p[k] -= lr * (mk / c1) / (sqrtf(vk / c2) + 1e-8f);
-}
-
-void launch_adam(float *params, float *m, float *v, const float *grad, int step, float lr, cudaStream_t st) {
+void launch_mlp_train_step(float *params, float *m, float *v, uint32_t *pack, const float *features, const float *esj,
+                           long long n, int n_eps, const float *eps_grid_dev, float eps_min, float eps_max,
+                           float *partial, float *loss, int step, float lr, cudaStream_t st) {
+    const int nb = grad_blocks(n);
     const float c1 = 1.f - powf(0.9f, (float)step), c2 = 1.f - powf(0.999f, (float)step);
-    k_adam<<<(kMlpParams + 255) / 256, 256, 0, st>>>(params, m, v, grad, lr, c1, c2);
+    launch_chained(k_mlp_grad, nb, 128, st, params, pack, features, esj, n, n_eps, eps_grid_dev, eps_min, eps_max,
+                   partial);
+    launch_chained(k_mlp_step<true>, (kGradSlots + 31) / 32, kStepThreads, st, partial, nb,
+                   static_cast<float *>(nullptr), loss, params, m, v, pack, lr, c1, c2);
 }
 
 }  // namespace glac
@@ -839,11 +934,9 @@ glac_status glac_mlp_train(glac_mlp *M, const float *dev_features, const float *
             const long long nb = n / batch;  // whole batches, cycled in order
             for (int it = 0; it < steps; it++) {
                 const long long off = (it % nb) * batch;
-                launch_mlp_grad(M->params, M->pack, dev_features + off * 8, dev_esj + off * n_eps, batch, n_eps,
-                                M->grid, (float)eps_grid[0], (float)eps_grid[n_eps - 1], M->partial, M->grad,
-                                loss_dev + it, M->stream);
-                launch_adam(M->params, M->m, M->v, M->grad, ++M->step, (float)lr, M->stream);
-                launch_mlp_pack(M->params, M->pack, M->stream);
+                launch_mlp_train_step(M->params, M->m, M->v, M->pack, dev_features + off * 8, dev_esj + off * n_eps,
+                                      batch, n_eps, M->grid, (float)eps_grid[0], (float)eps_grid[n_eps - 1],
+                                      M->partial, loss_dev + it, ++M->step, (float)lr, M->stream);
             }
             mck(cudaGetLastError(), "train");
             if (steps > 0)

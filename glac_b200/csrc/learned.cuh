@@ -213,6 +213,9 @@ size_t mlp_grad_scratch(long long n);
 void launch_mlp_grad(const float *params, const uint32_t *pack, const float *features, const float *esj, long long n,
                      int n_eps, const float *eps_grid_dev, float eps_min, float eps_max, float *partial, float *grad,
                      float *loss, cudaStream_t st);
-void launch_adam(float *params, float *m, float *v, const float *grad, int step, float lr, cudaStream_t st);
+// The gradient of one batch, then the Adam update of the parameters and their packed fragments (step counts from 1).
+void launch_mlp_train_step(float *params, float *m, float *v, uint32_t *pack, const float *features, const float *esj,
+                           long long n, int n_eps, const float *eps_grid_dev, float eps_min, float eps_max,
+                           float *partial, float *loss, int step, float lr, cudaStream_t st);
 
 }  // namespace glac

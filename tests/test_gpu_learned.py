@@ -173,6 +173,38 @@ def test_gradient_matches_oracle(g, torch, learned):
         assert np.linalg.norm(grad[a:b] - go[a:b]) < 0.02 * np.linalg.norm(go[a:b]) + 1e-7, (a, b)
 
 
+@pytest.mark.parametrize("n", [1, 16, 17, 64, 65, 18944, 18945])
+def test_train_step_is_adam_of_the_gradient(g, torch, learned, n):
+    # n around the edges of a 16-row tile, a four-tile block, and one tile to
+    # each warp of the largest grid (296 x 4 x 16 rows).  The step's sum, update
+    # and packing against the gradient entry point: the loss has the same bits;
+    # the first Adam step, done here in FP32, may differ by a few roundings of
+    # the update (at most lr) and one of the parameter; and the fragments the
+    # step packed give the spreads of a network that was given its parameters.
+    rng = np.random.default_rng(n)
+    grid = np.geomspace(0.03, 0.9, 16)
+    X = torch.from_numpy(rng.standard_normal((n, 8)).astype(np.float32)).cuda()
+    J = torch.from_numpy(rng.random((n, 16)).astype(np.float32)).cuda()
+    lr = np.float32(2e-3)
+    with learned.ProposalNet() as net, learned.ProposalNet() as other:
+        p0 = random_params(n)
+        net.params = p0
+        loss, grad = net.loss_grad(X, J, grid)
+        losses = net.train(X, J, grid, 1, n, float(lr))
+        p1 = net.params
+        assert losses[0] == loss
+        one = np.float32(1)
+        c1, c2 = one - np.float32(0.9), one - np.float32(0.999)
+        m, v = np.float32(0.1) * grad, np.float32(0.001) * grad * grad
+        want = p0 - lr * (m / c1) / (np.sqrt(v / c2) + np.float32(1e-8))
+        assert np.all(np.abs(p1 - want) <= 2.0 ** -20 * lr + 2.0 ** -23 * np.abs(p0))
+        other.params = p1
+        assert torch.equal(net.forward(X, 0.03, 0.9), other.forward(X, 0.03, 0.9))
+        a, ga = net.loss_grad(X, J, grid)
+        b, gb = other.loss_grad(X, J, grid)
+        assert a == b and np.array_equal(ga, gb)
+
+
 def test_training_finds_known_optimum(g, torch, learned):
     # J_i(eps) peaks at eps*(x_i) = 0.1 + 0.5 sigmoid(2 x_i0): the trained spread must follow it
     rng = np.random.default_rng(5)
