@@ -298,7 +298,8 @@ class Lattice:
 
     def flow_stage_times_measured(self, n_steps: int):
         """Seconds per launch of [stage 0 with the clover parts, the measurement's
-        reduction, stage 1, stage 2] over n_steps measured flow steps."""
+        combination where it is a pass of its own, stage 1, stage 2] over n_steps
+        measured flow steps."""
         out = np.zeros(4)
         self._ck(lib().glac_flow_stage_times_measured(self._ctx, int(n_steps), out))
         return out

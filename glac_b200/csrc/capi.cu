@@ -26,6 +26,8 @@ struct glac_ctx {
     double *partial4 = nullptr;  // SuperSampler partials, 4 per block (allocated on first use)
     double *obs_dev = nullptr;
     size_t obs_cap = 0;  // doubles in obs_dev
+    double *flow_partial = nullptr;  // partial sums of a flow's measurements (first measured flow)
+    size_t flow_partial_cap = 0;     // doubles
     unsigned long long *acc_dev = nullptr;
     double *staging = nullptr;
     double *scalar_dev = nullptr;
@@ -164,70 +166,107 @@ void reunit(glac_ctx *c) {
     c->launches += 1;
 }
 
+// How this context's flow steps run.
+struct FlowMode {
+    bool split;      // each link's staple terms over six warps (split.cu)
+    bool in_stage1;  // the measurement's combination inside stage 1, else a pass of its own
+    int nb;          // its partial sums per half time slice
+    size_t row;      // doubles of one measurement's partial sums
+};
+// The split stage where the lattice is small and nothing else was asked for by
+// option or tuning: up to one and a half times the thread slots of a link per
+// thread (148 SMs x 24 warps in FP32), in FP64 once (x 16 warps), beyond which
+// its idle warps cost more than its shorter chain gives.  Microseconds per
+// measured step on B200, split / a thread per link: FP32 8^3 x 16 16.9 / 22.0,
+// 12^3 x 24 57 / 60, 14^3 x 28 108 / 101; FP64 8^3 x 16 33 / 36, 10^3 x 20
+// 74 / 74, 12^3 x 24 125 / 120.
+constexpr int kSplitMaxSitesFp32 = 148 * 24 * 32 * 3 / 2 / 4, kSplitMaxSitesFp64 = 148 * 16 * 32 / 4;
+FlowMode flow_mode(const glac_ctx *c) {
+    FlowMode m;
+    const int fused_default = c->d.precision == GLAC_FP32 ? 2 : 1;
+    m.split = c->g.V <= (c->d.precision == GLAC_FP32 ? kSplitMaxSitesFp32 : kSplitMaxSitesFp64) &&
+              c->d.exp_func == GLAC_EXP_MORNINGSTAR && c->tune[FAM_FLOW] == 0 && c->fused_measure == fused_default;
+    m.in_stage1 = c->fused_combine && (m.split ? flow_split_combines(c->g) : obs_combine_in_stage1(c->g, c->plan));
+    m.nb = m.split && m.in_stage1 ? c->g.Vh / c->g.N[3] / 32 : c->plan.nb;
+    m.row = (size_t)6 * m.nb * c->g.N[3];
+    return m;
+}
+void ensure_flow_partial(glac_ctx *c, size_t n) {
+    if (c->flow_partial_cap >= n) return;
+    if (c->flow_partial) cudaFree(c->flow_partial);
+    c->flow_partial = nullptr;
+    c->flow_partial_cap = 0;
+    ck(cudaMalloc(&c->flow_partial, n * sizeof(double)), "cudaMalloc flow partials");
+    c->flow_partial_cap = n;
+}
+
+template <typename T> LinkField<T> link_field(glac_ctx *c, int i) {
+    if constexpr (sizeof(T) == 8) return f64(c, i);
+    else return f32(c, i);
+}
+template <typename T> ForceField<T> force_field(glac_ctx *c) {
+    if constexpr (sizeof(T) == 8) return z64(c);
+    else return z32(c);
+}
+
 // One Luscher RK3 step: three fused stages, cur -> other -> cur -> other.
 // ev (optional) receives 4 events around the three stage launches, 5 with
-// meas_out (the fourth after the measurement's reduction).  meas_out
-// (optional, device): the observables of the field before the step, measured
-// inside stage 0 (clover parts) and reduced right after it.
-void flow_step(glac_ctx *c, cudaEvent_t *ev = nullptr, double *meas_out = nullptr) {
+// partial (the fourth after the measurement's combination pass, if it has one).
+// partial (optional, device, mode.row): the partial sums of the
+// observables of the field before the step, measured inside stage 0 (clover
+// parts) and combined after it or in stage 1.
+template <typename T>
+void flow_step_t(glac_ctx *c, const FlowMode &mode, cudaEvent_t *ev, double *partial) {
     const double eps = c->d.flow_eps;
     const double alpha[3] = {eps * 0.25, eps * 0.8888888888888888, 0.75 * eps};
     const double beta[3] = {0.0, -(eps * 0.4722222222222222), -1.0};
     if (ev) ck(cudaEventRecord(ev[0], c->stream), "event");
     int e = 1;
-    // the measurement's per-site combination and reduction: folded into stage 1
-    // where the lattice's half time slices are whole 128-site blocks
-    const bool in_stage1 = meas_out && c->fused_combine && obs_combine_in_stage1(c->g, c->plan);
+    const ForceField<T> z = force_field<T>(c);
+    CloverParts<T> cp;
+    if (partial) {
+        ensure_clover(c);
+        cp = clover_view<T>(c);
+    }
     for (int stage = 0; stage < 3; stage++) {
         const int src = c->cur, dst = c->cur ^ 1;
-        if (stage == 1 && in_stage1) {
-            // the site-per-thread stage where the flow family's chosen variant has that shape
-            const bool site = variant_shape(FAM_FLOW, c->d.precision == GLAC_FP32, c->tune[FAM_FLOW]) == 3;
-            if (c->d.precision == GLAC_FP64)
-                launch_flow_stage1_combine(c->g, f64(c, src), f64(c, dst), z64(c), c->d.exp_func, alpha[1], beta[1],
-                                           clover_view<double>(c), c->plan, c->partial, meas_out, false, c->stream);
-            else
-                launch_flow_stage1_combine(c->g, f32(c, src), f32(c, dst), z32(c), c->d.exp_func, alpha[1], beta[1],
-                                           clover_view<float>(c), c->plan, c->partial, meas_out, site, c->stream);
-            ck_launch("flow stage 1 with the measurement's reduction");
-            c->launches += 2;
-        } else if (stage == 0 && meas_out) {
-            ensure_clover(c);
-            // 1: link per thread, compiler's registers; 2: the same capped at 128;
-            // 3 (FP32): site per thread, upper staple products shared; 4 (FP32):
-            // link per thread capped at 96 (five blocks per SM, small spill)
+        const LinkField<T> in = link_field<T>(c, src), out = link_field<T>(c, dst);
+        if (mode.split) {
+            const bool meas = partial && (stage == 0 || (stage == 1 && mode.in_stage1));
+            launch_flow_split(c->g, in, out, z, stage, alpha[stage], beta[stage], meas ? &cp : nullptr, partial,
+                              c->stream);
+        } else if (stage == 0 && partial) {
+            // 1: link per thread, compiler's registers (FP64: three blocks per SM); 2: the
+            // same capped at 128; 3 (FP32): site per thread, upper staple products shared; 4
+            // (FP32): link per thread capped at 96 (five blocks per SM, small spill)
             const int fm = c->fused_measure;
-            const int regs = fm == 2 ? 128 : fm == 3 ? 3 : fm == 4 ? 96 : 0;
-            if (c->d.precision == GLAC_FP64) {
-                const CloverParts<double> cp = clover_view<double>(c);
-                launch_flow_stage0_meas(c->g, f64(c, src), f64(c, dst), z64(c), cp, c->d.exp_func, alpha[0], regs,
-                                        c->stream);
-                ck_launch("flow stage 0 with measurement");
-                if (ev) ck(cudaEventRecord(ev[e++], c->stream), "event");
-                if (!in_stage1) launch_obs_combine(c->g, cp, c->plan, c->partial, meas_out, c->stream);
-            } else {
-                const CloverParts<float> cp = clover_view<float>(c);
-                launch_flow_stage0_meas(c->g, f32(c, src), f32(c, dst), z32(c), cp, c->d.exp_func, alpha[0], regs,
-                                        c->stream);
-                ck_launch("flow stage 0 with measurement");
-                if (ev) ck(cudaEventRecord(ev[e++], c->stream), "event");
-                if (!in_stage1) launch_obs_combine(c->g, cp, c->plan, c->partial, meas_out, c->stream);
-            }
-            ck_launch("measurement from clover parts");
-            c->launches += in_stage1 ? 1 : 3;
+            launch_flow_stage0_meas(c->g, in, out, z, cp, c->d.exp_func, alpha[0],
+                                    fm == 2 ? 128 : fm == 3 ? 3 : fm == 4 ? 96 : 0, c->stream);
+        } else if (stage == 1 && partial && mode.in_stage1) {
+            // the site-per-thread stage where the flow family's chosen variant has that shape
+            launch_flow_stage1_combine(c->g, in, out, z, c->d.exp_func, alpha[1], beta[1], cp, c->plan, partial,
+                                       variant_shape(FAM_FLOW, sizeof(T) == 4, c->tune[FAM_FLOW]) == 3, c->stream);
         } else {
-            if (c->d.precision == GLAC_FP64)
-                launch_flow_stage(c->g, f64(c, src), f64(c, dst), z64(c), stage, c->d.exp_func, alpha[stage],
-                                  beta[stage], c->tune[FAM_FLOW], c->stream);
-            else
-                launch_flow_stage(c->g, f32(c, src), f32(c, dst), z32(c), stage, c->d.exp_func, alpha[stage],
-                                  beta[stage], c->tune[FAM_FLOW], c->stream);
-            ck_launch("flow stage");
-            c->launches += 1;
+            launch_flow_stage(c->g, in, out, z, stage, c->d.exp_func, alpha[stage], beta[stage], c->tune[FAM_FLOW],
+                              c->stream);
+        }
+        ck_launch("flow stage");
+        c->launches += 1;
+        if (stage == 0 && partial) {
+            if (ev) ck(cudaEventRecord(ev[e++], c->stream), "event");
+            if (!mode.in_stage1) {
+                launch_obs_combine(c->g, cp, c->plan, partial, c->stream);
+                ck_launch("measurement from clover parts");
+                c->launches += 1;
+            }
         }
         c->cur = dst;
         if (ev) ck(cudaEventRecord(ev[e++], c->stream), "event");
     }
+}
+void flow_step(glac_ctx *c, const FlowMode &mode, cudaEvent_t *ev = nullptr, double *partial = nullptr) {
+    if (c->d.precision == GLAC_FP64) flow_step_t<double>(c, mode, ev, partial);
+    else flow_step_t<float>(c, mode, ev, partial);
 }
 
 glac_status need_field(glac_ctx *c) {
@@ -306,6 +345,7 @@ void glac_destroy(glac_ctx *c) {
     if (c->force) cudaFree(c->force);
     if (c->partial) cudaFree(c->partial);
     if (c->partial4) cudaFree(c->partial4);
+    if (c->flow_partial) cudaFree(c->flow_partial);
     if (c->obs_dev) cudaFree(c->obs_dev);
     if (c->acc_dev) cudaFree(c->acc_dev);
     if (c->staging) cudaFree(c->staging);
@@ -600,12 +640,26 @@ glac_status glac_flow(glac_ctx *c, int n_steps, double *obs) {
         // allows (the field it flows is the one to measure), else a pass of its
         // own; the last one always a pass of its own.
         const bool fused = obs && fused_measure_usable(c);
+        const FlowMode mode = flow_mode(c);
+        int rows = 1;  // measurements whose partial sums wait for one final reduction (16 MB at most)
         if (obs) {
             ensure_obs(c, per * (size_t)(n_steps + 1));
             if (!fused || n_steps == 0) measure_into(c, c->obs_dev);
+            if (fused && n_steps > 0) {
+                const size_t fit = ((size_t)16 << 20) / (mode.row * sizeof(double));
+                rows = fit < 1 ? 1 : fit > (size_t)n_steps ? n_steps : (int)fit;
+                ensure_flow_partial(c, rows * mode.row);
+            }
         }
         for (int i = 0; i < n_steps; i++) {
-            flow_step(c, nullptr, fused ? c->obs_dev + per * (size_t)i : nullptr);
+            const int r = i % rows;
+            flow_step(c, mode, nullptr, fused ? c->flow_partial + mode.row * (size_t)r : nullptr);
+            if (fused && (r == rows - 1 || i == n_steps - 1)) {
+                launch_obs_finalize(c->g, mode.nb, r + 1, c->flow_partial, c->obs_dev + per * (size_t)(i - r),
+                                    c->stream);
+                ck_launch("measurement reduction");
+                c->launches += 1;
+            }
             if (c->d.reunit_interval > 0 && c->d.precision == GLAC_FP32 && (i + 1) % c->d.reunit_interval == 0)
                 reunit(c);
             if (obs && (!fused || i == n_steps - 1)) measure_into(c, c->obs_dev + per * (size_t)(i + 1));
@@ -629,7 +683,7 @@ glac_status glac_flow_stage_times(glac_ctx *c, int n_steps, double *seconds3) {
         for (int i = 0; i < 4; i++) ck(cudaEventCreate(&ev[i]), "event create");
         double acc[3] = {0, 0, 0};
         for (int k = 0; k < n_steps; k++) {
-            flow_step(c, ev);
+            flow_step(c, flow_mode(c), ev);
             ck(cudaEventSynchronize(ev[3]), "event sync");
             for (int i = 0; i < 3; i++) {
                 float ms = 0.f;
@@ -653,13 +707,13 @@ glac_status glac_flow_stage_times_measured(glac_ctx *c, int n_steps, double *sec
                      "lattice is too large for the clover parts' 32-bit offsets)";
             return GLAC_ERR_STATE;
         }
-        const size_t per = 3 + (size_t)c->g.N[3];
-        ensure_obs(c, per);
+        const FlowMode mode = flow_mode(c);
+        ensure_flow_partial(c, mode.row);
         cudaEvent_t ev[5];
         for (int i = 0; i < 5; i++) ck(cudaEventCreate(&ev[i]), "event create");
         double acc[4] = {0, 0, 0, 0};
         for (int k = 0; k < n_steps; k++) {
-            flow_step(c, ev, c->obs_dev);
+            flow_step(c, mode, ev, c->flow_partial);
             ck(cudaEventSynchronize(ev[4]), "event sync");
             for (int i = 0; i < 4; i++) {
                 float ms = 0.f;
@@ -713,8 +767,11 @@ glac_status glac_autotune(glac_ctx *c, int reps, double *report) {
                         // flows measure after every step where the measurement runs
                         // inside the stages, so the flow family is timed on such steps
                         if (fam == FAM_FLOW) {
-                            if (fused_measure_usable(c)) flow_step(c, nullptr, c->obs_dev);
-                            else flow_step(c);
+                            const FlowMode mode = flow_mode(c);
+                            if (fused_measure_usable(c)) {
+                                ensure_flow_partial(c, mode.row);
+                                flow_step(c, mode, nullptr, c->flow_partial);
+                            } else flow_step(c, mode);
                         } else if (fam == FAM_METRO) {
                             for (int k = 0; k < 8; k++) {
                                 if (fp32)

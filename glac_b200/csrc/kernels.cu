@@ -2,6 +2,8 @@
 // fused clover observables with deterministic FP64 reductions, plus field
 // initialisation, reunitarisation and layout conversion.
 #include "kernels.cuh"
+#include "flow_body.cuh"
+#include "launch.cuh"
 #include "learned.cuh"
 
 #include <algorithm>
@@ -54,13 +56,6 @@ __device__ __forceinline__ int tiled_chunk(const Geom &g, int j) {
     return k + K * (z + g.N[2] * t);
 }
 
-// Force of a link from its staple sum.  FP64 forms only the part of U A that
-// enters; in FP32 at 80 registers the full product was the faster one.
-template <typename T> __device__ __forceinline__ AH8<T> flow_force(const M3<T> &U, const M3<T> &A) {
-    if constexpr (sizeof(T) == 4) return project_ah(mul(U, A));
-    else return project_ah_mul(U, A);
-}
-
 template <typename T, int KIND, int STAGE, int SHAPE>
 __device__ __forceinline__ void flow_stage_body(const Geom &g, const LinkField<T> &in, const LinkField<T> &out,
                                                 const ForceField<T> &zf, T alpha, T beta, int bx) {
@@ -74,21 +69,7 @@ __device__ __forceinline__ void flow_stage_body(const Geom &g, const LinkField<T
     M3<T> A = staple<T, false, true>(in, g, n, p, mu);
     const M3<T> U = in.load(mu, p, s);
     const AH8<T> Z = flow_force(U, A);
-    AH8<T> M;
-    if (STAGE == 0) {
-        M = ah_scale(alpha, Z);
-        zf.store(mu, p, s, Z);
-    } else {
-        const AH8<T> W = zf.load(mu, p, s);
-        M = ah_axpby(alpha, Z, beta, W);
-        if (STAGE == 1) zf.store(mu, p, s, M);
-    }
-    if (KIND == EXP_MORNINGSTAR) {
-        // U' = U + (exp(M) - 1) U: the small product first, one rounding at |U|
-        out.store(mu, p, s, mul_plus_right(expm_morningstar<T, true>(M), U));
-    } else {
-        out.store(mu, p, s, mul(expm<T>(KIND, M), U));
-    }
+    flow_update<T, KIND, STAGE>(U, Z, out, zf, alpha, beta, mu, p, s);
 }
 
 // Shape 3 (FP32): one thread per site, its four links in turn.  The upper
@@ -108,11 +89,6 @@ constexpr int kSiteBlock = 128;
 
 // MEAS (stage 0 only): also the measurement's clover parts of the planes each
 // link direction takes, as flow_stage0_meas_body does (defined further down).
-__device__ __forceinline__ bool meas_takes(int mu, int nu);
-__host__ __device__ constexpr int plane_of(int a, int b);
-template <typename T> __device__ __forceinline__ AH8<T> proj_ah8(const M3<T> &C);
-template <typename T> __device__ __forceinline__ AH8<T> ah_neg_if(const AH8<T> &F, bool neg);
-
 template <typename T, int KIND, int STAGE, bool MEAS = false>
 __device__ __forceinline__ void flow_stage_site_body(const Geom &g, const LinkField<T> &in, const LinkField<T> &out,
                                                      const ForceField<T> &zf, T alpha, T beta, int bx, T *slots,
@@ -223,6 +199,7 @@ template <typename T, int KIND, int STAGE>
 __global__ void __launch_bounds__(kSiteBlock) k_flow_stage_site(Geom g, LinkField<T> in, LinkField<T> out,
                                                                 ForceField<T> zf, T alpha, T beta) {
     __shared__ T slots[4 * 18 * kSiteBlock];
+    chain_wait();
     flow_stage_site_body<T, KIND, STAGE>(g, in, out, zf, alpha, beta, blockIdx.x, slots);
 }
 
@@ -233,6 +210,7 @@ __global__ void __launch_bounds__(kSiteBlock) k_flow_stage_site(Geom g, LinkFiel
     template <typename T, int KIND, int STAGE, int SHAPE>                                                \
     __global__ void ATTR NAME(Geom g, LinkField<T> in, LinkField<T> out, ForceField<T> zf, T alpha,      \
                               T beta) {                                                                  \
+        chain_wait();                                                                                    \
         flow_stage_body<T, KIND, STAGE, SHAPE>(g, in, out, zf, alpha, beta, blockIdx.x);                 \
     }
 GLAC_FLOW_KERNEL(k_flow_stage, __launch_bounds__(128))
@@ -273,20 +251,20 @@ static void flow_dispatch_caps(int regs, cudaStream_t st, const Geom &g, const L
                                const LinkField<T> &out, const ForceField<T> &zf, T a, T b) {
     const dim3 grid(8 * ((g.Vh + 127) / 128));
     switch (regs) {
-    case 128: k_flow_stage_r128<T, KIND, STAGE, SHAPE><<<grid, 128, 0, st>>>(g, in, out, zf, a, b); break;
+    case 128: launch_chained(k_flow_stage_r128<T, KIND, STAGE, SHAPE>, grid.x, 128, st, g, in, out, zf, a, b); break;
     case 96:
         if constexpr (sizeof(T) == 4) {
-            k_flow_stage_r96<T, KIND, STAGE, SHAPE><<<grid, 128, 0, st>>>(g, in, out, zf, a, b);
+            launch_chained(k_flow_stage_r96<T, KIND, STAGE, SHAPE>, grid.x, 128, st, g, in, out, zf, a, b);
             break;
         }
         [[fallthrough]];
     case 80:
         if constexpr (sizeof(T) == 4) {
-            k_flow_stage_r80<T, KIND, STAGE, SHAPE><<<grid, 128, 0, st>>>(g, in, out, zf, a, b);
+            launch_chained(k_flow_stage_r80<T, KIND, STAGE, SHAPE>, grid.x, 128, st, g, in, out, zf, a, b);
             break;
         }
         [[fallthrough]];  // no 80-register FP64 variant
-    default: k_flow_stage<T, KIND, STAGE, SHAPE><<<grid, 128, 0, st>>>(g, in, out, zf, a, b); break;
+    default: launch_chained(k_flow_stage<T, KIND, STAGE, SHAPE>, grid.x, 128, st, g, in, out, zf, a, b); break;
     }
 }
 
@@ -296,13 +274,13 @@ static void flow_dispatch(int regs, int shape, cudaStream_t st, const Geom &g, c
     if constexpr (sizeof(T) == 4) {
         if (shape == 3) {
             const dim3 grid(2 * ((g.Vh + kSiteBlock - 1) / kSiteBlock));
-            k_flow_stage_site<T, KIND, STAGE><<<grid, kSiteBlock, 0, st>>>(g, in, out, zf, a, b);
+            launch_chained(k_flow_stage_site<T, KIND, STAGE>, grid.x, kSiteBlock, st, g, in, out, zf, a, b);
             return;
         }
     }
     if (shape == 1) {
         const dim3 grid((g.Vh + 15) / 16);
-        k_flow_stage<T, KIND, STAGE, 1><<<grid, 128, 0, st>>>(g, in, out, zf, a, b);
+        launch_chained(k_flow_stage<T, KIND, STAGE, 1>, grid.x, 128, st, g, in, out, zf, a, b);
         return;
     }
     if (shape == 2) flow_dispatch_caps<T, KIND, STAGE, 2>(regs, st, g, in, out, zf, a, b);
@@ -323,7 +301,7 @@ void launch_flow_stage(const Geom &g, const LinkField<T> &in, const LinkField<T>
         return;
     }
 #define GLAC_FLOW_CASE(K, S) \
-    if (kind == K && stage == S) { k_flow_stage<T, K, S, 0><<<grid, 128, 0, st>>>(g, in, out, zf, a, b); return; }
+    if (kind == K && stage == S) { launch_chained(k_flow_stage<T, K, S, 0>, grid.x, 128, st, g, in, out, zf, a, b); return; }
     GLAC_FLOW_CASE(1, 0) GLAC_FLOW_CASE(1, 1) GLAC_FLOW_CASE(1, 2)
     GLAC_FLOW_CASE(2, 0) GLAC_FLOW_CASE(2, 1) GLAC_FLOW_CASE(2, 2)
     GLAC_FLOW_CASE(3, 0) GLAC_FLOW_CASE(3, 1) GLAC_FLOW_CASE(3, 2)
@@ -356,48 +334,6 @@ template void launch_flow_stage<float>(const Geom &, const LinkField<float> &, c
 // plaquette slot.  k_obs_combine then adds the two slots of each plane per
 // site and reduces plaquette, Q(t) and E exactly as the observables kernel.
 // ---------------------------------------------------------------------------
-// (C - C^+) made traceless, in the 8-real form: diagonal 2 i Im C_ii minus a
-// third of its trace, off-diagonal C_ij - conj(C_ji).  Linear in C.
-template <typename T> __device__ __forceinline__ AH8<T> proj_ah8(const M3<T> &C) {
-    AH8<T> F;
-    const T two = T(2);
-    const T tr = (C(0, 0).im + C(1, 1).im + C(2, 2).im) * T(2.0 / 3.0);
-    F.a = two * C(0, 0).im - tr;
-    F.d = two * C(1, 1).im - tr;
-    F.b = cx(C(0, 1).re - C(1, 0).re, C(0, 1).im + C(1, 0).im);
-    F.c = cx(C(0, 2).re - C(2, 0).re, C(0, 2).im + C(2, 0).im);
-    F.e = cx(C(1, 2).re - C(2, 1).re, C(1, 2).im + C(2, 1).im);
-    return F;
-}
-template <typename T> __device__ __forceinline__ AH8<T> ah_add(const AH8<T> &X, const AH8<T> &Y) {
-    AH8<T> Z;
-    Z.a = X.a + Y.a;
-    Z.d = X.d + Y.d;
-    Z.b = X.b + Y.b;
-    Z.c = X.c + Y.c;
-    Z.e = X.e + Y.e;
-    return Z;
-}
-
-// plane index of (a, b), a < b: 01 0, 02 1, 03 2, 12 3, 13 4, 23 5
-__host__ __device__ constexpr int plane_of(int a, int b) { return a == 0 ? b - 1 : (a == 1 ? b + 1 : 5); }
-// the planes link direction mu takes (nu, or -1)
-__device__ __forceinline__ bool meas_takes(int mu, int nu) {
-    return (mu == 0 && (nu == 1 || nu == 2)) || (mu == 1 && (nu == 2 || nu == 3)) || (mu == 2 && nu == 3) ||
-           (mu == 3 && nu == 0);
-}
-
-template <typename T> __device__ __forceinline__ AH8<T> ah_neg_if(const AH8<T> &F, bool neg) {
-    return neg ? ah_scale(T(-1), F) : F;
-}
-
-// P(A B), negated where neg: twice project_ah of the product, with its sign turned
-// (FP64; FP32 forms the product, as flow_force).
-template <typename T> __device__ __forceinline__ AH8<T> clover_part(const M3<T> &A, const M3<T> &B, bool neg) {
-    if constexpr (sizeof(T) == 4) return ah_neg_if(proj_ah8(mul(A, B)), neg);
-    else return ah_scale(neg ? T(2) : T(-2), project_ah_mul(A, B));
-}
-
 template <typename T, int KIND>
 __device__ __forceinline__ void flow_stage0_meas_body(const Geom &g, const LinkField<T> &in, const LinkField<T> &out,
                                                       const ForceField<T> &zf, const CloverParts<T> &cp, T alpha,
@@ -453,17 +389,14 @@ __device__ __forceinline__ void flow_stage0_meas_body(const Geom &g, const LinkF
     }
     cp.plaq[(mu * 2 + p) * g.Vh + s] = plaq;
     const M3<T> U = in.load(mu, p, s);
-    const AH8<T> Z = flow_force(U, A);
-    zf.store(mu, p, s, Z);
-    const AH8<T> M = ah_scale(alpha, Z);
-    if (KIND == EXP_MORNINGSTAR) out.store(mu, p, s, mul_plus_right(expm_morningstar<T, true>(M), U));
-    else out.store(mu, p, s, mul(expm<T>(KIND, M), U));
+    flow_update<T, KIND, 0>(U, flow_force(U, A), out, zf, alpha, T(0), mu, p, s);
 }
 
 #define GLAC_FLOW_MEAS_KERNEL(NAME, ATTR)                                                                  \
     template <typename T, int KIND>                                                                      \
     __global__ void ATTR NAME(Geom g, LinkField<T> in, LinkField<T> out, ForceField<T> zf,               \
                               CloverParts<T> cp, T alpha) {                                              \
+        chain_wait();                                                                                    \
         flow_stage0_meas_body<T, KIND>(g, in, out, zf, cp, alpha, blockIdx.x);                           \
     }
 GLAC_FLOW_MEAS_KERNEL(k_flow_stage0_meas, __launch_bounds__(128))
@@ -479,6 +412,7 @@ template <typename T, int KIND>
 __global__ void __launch_bounds__(kSiteBlock) k_flow_stage0_meas_site(Geom g, LinkField<T> in, LinkField<T> out,
                                                                       ForceField<T> zf, CloverParts<T> cp, T alpha) {
     __shared__ T slots[4 * 18 * kSiteBlock];
+    chain_wait();
     flow_stage_site_body<T, KIND, 0, true>(g, in, out, zf, alpha, T(0), blockIdx.x, slots, &cp);
 }
 
@@ -486,12 +420,12 @@ template <typename T, int KIND>
 static void meas_dispatch(int regs, dim3 grid, cudaStream_t st, const Geom &g, const LinkField<T> &in,
                           const LinkField<T> &out, const ForceField<T> &zf, const CloverParts<T> &cp, T a) {
     if (regs == 128) {
-        k_flow_stage0_meas_r128<T, KIND><<<grid, 128, 0, st>>>(g, in, out, zf, cp, a);
+        launch_chained(k_flow_stage0_meas_r128<T, KIND>, grid.x, 128, st, g, in, out, zf, cp, a);
         return;
     }
-    if constexpr (sizeof(T) == 8) k_flow_stage0_meas_b3<T, KIND><<<grid, 128, 0, st>>>(g, in, out, zf, cp, a);
-    else if (regs == 96) k_flow_stage0_meas_r96<T, KIND><<<grid, 128, 0, st>>>(g, in, out, zf, cp, a);
-    else k_flow_stage0_meas<T, KIND><<<grid, 128, 0, st>>>(g, in, out, zf, cp, a);
+    if constexpr (sizeof(T) == 8) launch_chained(k_flow_stage0_meas_b3<T, KIND>, grid.x, 128, st, g, in, out, zf, cp, a);
+    else if (regs == 96) launch_chained(k_flow_stage0_meas_r96<T, KIND>, grid.x, 128, st, g, in, out, zf, cp, a);
+    else launch_chained(k_flow_stage0_meas<T, KIND>, grid.x, 128, st, g, in, out, zf, cp, a);
 }
 
 template <typename T>
@@ -503,10 +437,10 @@ void launch_flow_stage0_meas(const Geom &g, const LinkField<T> &in, const LinkFi
         if (regs == 3) {  // the site-per-thread form
             const dim3 gs(2 * ((g.Vh + kSiteBlock - 1) / kSiteBlock));
             switch (kind) {
-            case 0: k_flow_stage0_meas_site<T, 0><<<gs, kSiteBlock, 0, st>>>(g, in, out, zf, cp, a); return;
-            case 1: k_flow_stage0_meas_site<T, 1><<<gs, kSiteBlock, 0, st>>>(g, in, out, zf, cp, a); return;
-            case 2: k_flow_stage0_meas_site<T, 2><<<gs, kSiteBlock, 0, st>>>(g, in, out, zf, cp, a); return;
-            case 3: k_flow_stage0_meas_site<T, 3><<<gs, kSiteBlock, 0, st>>>(g, in, out, zf, cp, a); return;
+            case 0: launch_chained(k_flow_stage0_meas_site<T, 0>, gs.x, kSiteBlock, st, g, in, out, zf, cp, a); return;
+            case 1: launch_chained(k_flow_stage0_meas_site<T, 1>, gs.x, kSiteBlock, st, g, in, out, zf, cp, a); return;
+            case 2: launch_chained(k_flow_stage0_meas_site<T, 2>, gs.x, kSiteBlock, st, g, in, out, zf, cp, a); return;
+            case 3: launch_chained(k_flow_stage0_meas_site<T, 3>, gs.x, kSiteBlock, st, g, in, out, zf, cp, a); return;
             default: throw std::invalid_argument("bad exp kind");
             }
         }
@@ -705,6 +639,7 @@ __device__ __forceinline__ unsigned long long metropolis_hits(const LinkField<T>
             na++;
         }
     }
+    chain_release();
     L.store(mu, p, s, U);
     return na;
 }
@@ -750,6 +685,7 @@ __device__ __forceinline__ void metropolis_body(const Geom &g, const LinkField<T
     __global__ void ATTR NAME(Geom g, LinkField<T> L, int mu, int p, T mfac, T eps, T sq1me, int nhits,      \
                               uint32_t k0, uint32_t k1, uint32_t sweep, uint32_t stream_id,                 \
                               unsigned long long *acc, Proposal P, float beta) {                            \
+        chain_wait();                                                                                     \
         metropolis_body<T, LEARNED>(g, L, mu, p, mfac, eps, sq1me, nhits, k0, k1, sweep, stream_id, acc, P,  \
                                     beta, blockIdx.x);                                                     \
     }
@@ -764,10 +700,10 @@ static void metro_dispatch(int regs, dim3 grid, cudaStream_t st, const Geom &g, 
                            int p, T mfac, T e, T sq, int nhits, uint32_t k0, uint32_t k1, uint32_t sweep,
                            uint32_t stream_id, unsigned long long *acc, const Proposal &P, float beta) {
     switch (regs) {
-    case 128: k_metropolis_r128<T, LEARNED><<<grid, 128, 0, st>>>(g, L, mu, p, mfac, e, sq, nhits, k0, k1, sweep, stream_id, acc, P, beta); break;
-    case 96: k_metropolis_r96<T, LEARNED><<<grid, 128, 0, st>>>(g, L, mu, p, mfac, e, sq, nhits, k0, k1, sweep, stream_id, acc, P, beta); break;
-    case 80: k_metropolis_r80<T, LEARNED><<<grid, 128, 0, st>>>(g, L, mu, p, mfac, e, sq, nhits, k0, k1, sweep, stream_id, acc, P, beta); break;
-    default: k_metropolis<T, LEARNED><<<grid, 128, 0, st>>>(g, L, mu, p, mfac, e, sq, nhits, k0, k1, sweep, stream_id, acc, P, beta); break;
+    case 128: launch_chained(k_metropolis_r128<T, LEARNED>, grid.x, 128, st, g, L, mu, p, mfac, e, sq, nhits, k0, k1, sweep, stream_id, acc, P, beta); break;
+    case 96: launch_chained(k_metropolis_r96<T, LEARNED>, grid.x, 128, st, g, L, mu, p, mfac, e, sq, nhits, k0, k1, sweep, stream_id, acc, P, beta); break;
+    case 80: launch_chained(k_metropolis_r80<T, LEARNED>, grid.x, 128, st, g, L, mu, p, mfac, e, sq, nhits, k0, k1, sweep, stream_id, acc, P, beta); break;
+    default: launch_chained(k_metropolis<T, LEARNED>, grid.x, 128, st, g, L, mu, p, mfac, e, sq, nhits, k0, k1, sweep, stream_id, acc, P, beta); break;
     }
 }
 
@@ -979,26 +915,6 @@ __device__ __forceinline__ AH8<T> clover_ah(const LinkField<T> &L, const Geom &g
     else return clover_ah_call<T>(L, g, n, p, mu, nu, plaq);
 }
 
-// Re Tr(F G) for traceless anti-Hermitian F, G in the 8-real form:
-//   -[a a' + d d' + (a+d)(a'+d')] - 2 Re(b b'* + c c'* + e e'*)
-template <typename T>
-__device__ __forceinline__ T retr_ah(const AH8<T> &F, const AH8<T> &G) {
-    T diag = fmaR(F.a, G.a, F.d * G.d);
-    diag = fmaR(F.a + F.d, G.a + G.d, diag);
-    T off = fmaR(F.b.re, G.b.re, F.b.im * G.b.im);
-    off = fmaR(F.c.re, G.c.re, off);
-    off = fmaR(F.c.im, G.c.im, off);
-    off = fmaR(F.e.re, G.e.re, off);
-    off = fmaR(F.e.im, G.e.im, off);
-    return -(diag + off + off);
-}
-
-__device__ __forceinline__ double warp_sum_d(double v) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
-    return v;
-}
-
 // Block sums of the three per-thread values in a fixed order (warp shuffles,
 // then the warps in order) into partial[3 b .. 3 b + 2] = (plaq, energy, q).
 __device__ __forceinline__ void obs_block_reduce(double plaq, double en, double qt, double *partial, int b) {
@@ -1100,8 +1016,13 @@ __device__ __forceinline__ void obs_finalize_body(int Nt, int nb, int V, const d
         for (int t = 0; t < Nt; t++) out[3 + t] = sq[t] * qfac;
     }
 }
+// One measurement per block: rows of 3 (2 nb Nt) partials in, rows of 3 + Nt out.
 __global__ void k_obs_finalize(int Nt, int nb, int V, const double *partial, double *out) {
-    obs_finalize_body(Nt, nb, V, partial, out);
+    obs_finalize_body(Nt, nb, V, partial + (size_t)blockIdx.x * 6 * nb * Nt, out + (size_t)blockIdx.x * (3 + Nt));
+}
+void launch_obs_finalize(const Geom &g, int nb, int rows, const double *partial, double *out, cudaStream_t st) {
+    if (g.N[3] > 1024) throw std::invalid_argument("Nt > 1024 not supported by the observable reduction");
+    k_obs_finalize<<<rows, 1024, 0, st>>>(g.N[3], nb, g.V, partial, out);
 }
 
 template <typename T>
@@ -1125,20 +1046,6 @@ void launch_observables(const Geom &g, const LinkField<T> &L, const ObsPlan &pla
 // per site F of each plane = its local + forward slot, the plaquette = the four
 // direction sums; Q(t), E and the plaquette reduced as in observables_body (same
 // blocks, same fixed order), then k_obs_finalize.
-template <typename T>
-__device__ __forceinline__ void combine_site(const Geom &g, const CloverParts<T> &cp, int p, int s, double &plaq,
-                                             double &en, double &qt) {
-    AH8<T> F[6];
-#pragma unroll
-    for (int pl = 0; pl < 6; pl++) F[pl] = ah_add(cp.ah.load(2 * pl, p, s), cp.ah.load(2 * pl + 1, p, s));
-#pragma unroll
-    for (int mu = 0; mu < 4; mu++) plaq += (double)cp.plaq[(mu * 2 + p) * g.Vh + s];
-    // q = -[ReTr(F_01 F_23) + ReTr(F_02 F_31) + ReTr(F_03 F_12)], F_31 = -F_13
-    qt = -((double)retr_ah(F[0], F[5]) - (double)retr_ah(F[1], F[4]) + (double)retr_ah(F[2], F[3]));
-#pragma unroll
-    for (int pl = 0; pl < 6; pl++) en += (double)retr_ah(F[pl], F[pl]);
-}
-
 template <typename T>
 __global__ void __launch_bounds__(256) k_obs_combine(Geom g, CloverParts<T> cp, int nb, int Bv, double *partial) {
     const int b = blockIdx.x;
@@ -1166,6 +1073,7 @@ template <typename T, int KIND>
 __global__ void __launch_bounds__(128, sizeof(T) == 4 ? 6 : 4) k_flow_stage1_combine(Geom g, LinkField<T> in, LinkField<T> out,
                                                              ForceField<T> zf, T alpha, T beta, CloverParts<T> cp,
                                                              double *partial) {
+    chain_wait();
     flow_stage_body<T, KIND, 1, 0>(g, in, out, zf, alpha, beta, blockIdx.x);
     const int plane = blockIdx.x & 7;
     if (plane >= 2) return;  // a whole block returns together
@@ -1187,6 +1095,7 @@ __global__ void __launch_bounds__(kSiteBlock) k_flow_stage1_combine_site(Geom g,
                                                                          ForceField<T> zf, T alpha, T beta,
                                                                          CloverParts<T> cp, double *partial) {
     __shared__ T slots[4 * 18 * kSiteBlock];
+    chain_wait();
     flow_stage_site_body<T, KIND, 1>(g, in, out, zf, alpha, beta, blockIdx.x, slots);
     const int p = blockIdx.x & 1;
     const int s0 = (blockIdx.x >> 1) * kSiteBlock, s = s0 + threadIdx.x;
@@ -1206,9 +1115,8 @@ bool obs_combine_in_stage1(const Geom &g, const ObsPlan &plan) {
 template <typename T>
 void launch_flow_stage1_combine(const Geom &g, const LinkField<T> &in, const LinkField<T> &out,
                                 const ForceField<T> &zf, int kind, double alpha, double beta,
-                                const CloverParts<T> &cp, const ObsPlan &plan, double *partial, double *obs_out,
-                                bool site, cudaStream_t st) {
-    if (g.N[3] > 1024) throw std::invalid_argument("Nt > 1024 not supported by the observable reduction");
+                                const CloverParts<T> &cp, const ObsPlan &plan, double *partial, bool site,
+                                cudaStream_t st) {
     if (!obs_combine_in_stage1(g, plan)) throw std::invalid_argument("lattice does not allow the stage-1 combine");
     const dim3 grid(8 * (g.Vh / 128));
     const T a = (T)alpha, b = (T)beta;
@@ -1216,44 +1124,40 @@ void launch_flow_stage1_combine(const Geom &g, const LinkField<T> &in, const Lin
         if (site) {
             const dim3 gs(2 * (g.Vh / kSiteBlock));
             switch (kind) {
-            case 0: k_flow_stage1_combine_site<T, 0><<<gs, kSiteBlock, 0, st>>>(g, in, out, zf, a, b, cp, partial); break;
-            case 1: k_flow_stage1_combine_site<T, 1><<<gs, kSiteBlock, 0, st>>>(g, in, out, zf, a, b, cp, partial); break;
-            case 2: k_flow_stage1_combine_site<T, 2><<<gs, kSiteBlock, 0, st>>>(g, in, out, zf, a, b, cp, partial); break;
-            case 3: k_flow_stage1_combine_site<T, 3><<<gs, kSiteBlock, 0, st>>>(g, in, out, zf, a, b, cp, partial); break;
+            case 0: launch_chained(k_flow_stage1_combine_site<T, 0>, gs.x, kSiteBlock, st, g, in, out, zf, a, b, cp, partial); break;
+            case 1: launch_chained(k_flow_stage1_combine_site<T, 1>, gs.x, kSiteBlock, st, g, in, out, zf, a, b, cp, partial); break;
+            case 2: launch_chained(k_flow_stage1_combine_site<T, 2>, gs.x, kSiteBlock, st, g, in, out, zf, a, b, cp, partial); break;
+            case 3: launch_chained(k_flow_stage1_combine_site<T, 3>, gs.x, kSiteBlock, st, g, in, out, zf, a, b, cp, partial); break;
             default: throw std::invalid_argument("bad exp kind");
             }
-            k_obs_finalize<<<1, 1024, 0, st>>>(g.N[3], plan.nb, g.V, partial, obs_out);
             return;
         }
     }
     switch (kind) {
-    case 0: k_flow_stage1_combine<T, 0><<<grid, 128, 0, st>>>(g, in, out, zf, a, b, cp, partial); break;
-    case 1: k_flow_stage1_combine<T, 1><<<grid, 128, 0, st>>>(g, in, out, zf, a, b, cp, partial); break;
-    case 2: k_flow_stage1_combine<T, 2><<<grid, 128, 0, st>>>(g, in, out, zf, a, b, cp, partial); break;
-    case 3: k_flow_stage1_combine<T, 3><<<grid, 128, 0, st>>>(g, in, out, zf, a, b, cp, partial); break;
+    case 0: launch_chained(k_flow_stage1_combine<T, 0>, grid.x, 128, st, g, in, out, zf, a, b, cp, partial); break;
+    case 1: launch_chained(k_flow_stage1_combine<T, 1>, grid.x, 128, st, g, in, out, zf, a, b, cp, partial); break;
+    case 2: launch_chained(k_flow_stage1_combine<T, 2>, grid.x, 128, st, g, in, out, zf, a, b, cp, partial); break;
+    case 3: launch_chained(k_flow_stage1_combine<T, 3>, grid.x, 128, st, g, in, out, zf, a, b, cp, partial); break;
     default: throw std::invalid_argument("bad exp kind");
     }
-    k_obs_finalize<<<1, 1024, 0, st>>>(g.N[3], plan.nb, g.V, partial, obs_out);
 }
 template void launch_flow_stage1_combine<double>(const Geom &, const LinkField<double> &, const LinkField<double> &,
                                                  const ForceField<double> &, int, double, double,
-                                                 const CloverParts<double> &, const ObsPlan &, double *, double *,
-                                                 bool, cudaStream_t);
+                                                 const CloverParts<double> &, const ObsPlan &, double *, bool,
+                                                 cudaStream_t);
 template void launch_flow_stage1_combine<float>(const Geom &, const LinkField<float> &, const LinkField<float> &,
                                                 const ForceField<float> &, int, double, double,
-                                                const CloverParts<float> &, const ObsPlan &, double *, double *,
-                                                bool, cudaStream_t);
+                                                const CloverParts<float> &, const ObsPlan &, double *, bool,
+                                                cudaStream_t);
 
 template <typename T>
-void launch_obs_combine(const Geom &g, const CloverParts<T> &cp, const ObsPlan &plan, double *partial, double *out,
+void launch_obs_combine(const Geom &g, const CloverParts<T> &cp, const ObsPlan &plan, double *partial,
                         cudaStream_t st) {
-    if (g.N[3] > 1024) throw std::invalid_argument("Nt > 1024 not supported by the observable reduction");
     k_obs_combine<T><<<plan.nblocks, plan.B, 0, st>>>(g, cp, plan.nb, plan.Bv, partial);
-    k_obs_finalize<<<1, 1024, 0, st>>>(g.N[3], plan.nb, g.V, partial, out);
 }
 template void launch_obs_combine<double>(const Geom &, const CloverParts<double> &, const ObsPlan &, double *,
-                                         double *, cudaStream_t);
-template void launch_obs_combine<float>(const Geom &, const CloverParts<float> &, const ObsPlan &, double *, double *,
+                                         cudaStream_t);
+template void launch_obs_combine<float>(const Geom &, const CloverParts<float> &, const ObsPlan &, double *,
                                         cudaStream_t);
 
 template <typename T>

@@ -99,21 +99,32 @@ void launch_flow_stage(const Geom &g, const LinkField<T> &in, const LinkField<T>
                        int stage, int kind, double alpha, double beta, int variant, cudaStream_t st);
 // Flow stage 0 that also writes the clover parts of its input field's
 // measurement (regs: 0 = the compiler's allocation, 128 = capped), and the
-// measurement from those parts ([plaq, topc, energy, topct[Nt]] into out).
+// measurement's block sums from those parts.
 template <typename T>
 void launch_flow_stage0_meas(const Geom &g, const LinkField<T> &in, const LinkField<T> &out, const ForceField<T> &zf,
                              const CloverParts<T> &cp, int kind, double alpha, int regs, cudaStream_t st);
 template <typename T>
-void launch_obs_combine(const Geom &g, const CloverParts<T> &cp, const ObsPlan &plan, double *partial, double *out,
+void launch_obs_combine(const Geom &g, const CloverParts<T> &cp, const ObsPlan &plan, double *partial,
                         cudaStream_t st);
-// Flow stage 1 with the measurement's combination and reduction folded in
-// (where obs_combine_in_stage1 holds), then the final reduction into obs_out.
+// `rows` measurements from their partial sums (6 nb Nt doubles each) into rows of [plaq, topc, energy, topct[Nt]].
+void launch_obs_finalize(const Geom &g, int nb, int rows, const double *partial, double *out, cudaStream_t st);
+// Flow stage 1 with the measurement's combination and block reduction folded in
+// (where obs_combine_in_stage1 holds).
 bool obs_combine_in_stage1(const Geom &g, const ObsPlan &plan);
 template <typename T>
 void launch_flow_stage1_combine(const Geom &g, const LinkField<T> &in, const LinkField<T> &out,
                                 const ForceField<T> &zf, int kind, double alpha, double beta,
-                                const CloverParts<T> &cp, const ObsPlan &plan, double *partial, double *obs_out,
-                                bool site, cudaStream_t st);
+                                const CloverParts<T> &cp, const ObsPlan &plan, double *partial, bool site,
+                                cudaStream_t st);
+// A Morningstar flow stage with each link's six staple terms on six warps
+// (split.cu).  With meas, stage 0 also writes the clover parts and stage 1
+// combines them (where flow_split_combines holds) into the partial sums of a
+// plan of 32-site blocks, nb = V / (64 Nt).
+bool flow_split_combines(const Geom &g);
+template <typename T>
+void launch_flow_split(const Geom &g, const LinkField<T> &in, const LinkField<T> &out, const ForceField<T> &zf,
+                       int stage, double alpha, double beta, const CloverParts<T> *meas, double *partial,
+                       cudaStream_t st);
 // whether the 12 clover-part slots of a lattice fit 32-bit element offsets
 inline bool clover_offsets_fit(long long V, bool fp64) {
     const long long vh32 = ((V / 2) + 31) / 32 * 32;

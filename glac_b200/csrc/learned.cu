@@ -15,6 +15,7 @@
 // fixed order, so the gradient is deterministic for a given n.
 #include "../../include/glac_b200.h"
 #include "learned.cuh"
+#include "launch.cuh"
 
 #include <cuda_runtime.h>
 
@@ -359,8 +360,8 @@ __device__ __forceinline__ uint2 ld_pack(const uint32_t *p) {
 }
 
 // With one tile to a warp (batches up to 18,944 rows) the pass is a chain of
-// load latencies, so what does not depend on the last step's parameters (rows,
-// grid) is fetched before the wait for it, and the fragments together after it.
+// load latencies, so what does not depend on the last step's parameters (its rows) is
+// fetched before the wait for it, and the fragments together after it.
 __global__ void __launch_bounds__(128) k_mlp_grad(const float *P, const uint32_t *pack,
                                                   const float *__restrict__ feat, const float *__restrict__ esj,
                                                   long long n, int n_eps, const float *__restrict__ eps_grid,
@@ -383,12 +384,12 @@ __global__ void __launch_bounds__(128) k_mlp_grad(const float *P, const uint32_t
             prefetch_l1(esj + r1 * n_eps + min(32 * t, n_eps - 1));
         }
     };
-    // none of this is written by the step before, so it may run beside its end
-    for (int k = threadIdx.x; k < n_eps; k += blockDim.x) grid_s[k] = eps_grid[k];
+    // the caller's rows are not written by the step before, so they may come in beside its end
     float2 x0, x1;
     fetch((long long)blockIdx.x * kGradWarps + warp, x0, x1);
-    cudaTriggerProgrammaticLaunchCompletion();
-    cudaGridDependencySynchronize();
+    chain_release();
+    chain_wait();
+    for (int k = threadIdx.x; k < n_eps; k += blockDim.x) grid_s[k] = eps_grid[k];
     __syncthreads();
     const float inv_n = 1.f / (float)n, span = eps_max - eps_min;
     const uint32_t one = t == 0 ? pack_bf16(1.f, 0.f) : 0u;
@@ -603,8 +604,8 @@ __global__ void __launch_bounds__(kStepThreads) k_mlp_step(const float *partial,
                                                            float c1, float c2) {
     __shared__ float rows[kGradMaxBlocks][32];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, k = blockIdx.x * 32 + lane;
-    cudaTriggerProgrammaticLaunchCompletion();
-    cudaGridDependencySynchronize();
+    chain_release();
+    chain_wait();
 #pragma unroll 8
     for (int b = warp; b < nblocks; b += kStepThreads / 32)
         rows[b][lane] = k < kGradSlots ? partial[(long long)b * kGradSlots + k] : 0.f;
@@ -638,22 +639,6 @@ static int grad_blocks(long long n) {
 }
 
 size_t mlp_grad_scratch(long long n) { return (size_t)grad_blocks(n) * kGradSlots; }
-
-// Launch that may start while the kernel before it drains (both wait for its
-// end, by cudaGridDependencySynchronize, before they touch what it writes).
-template <typename... Params, typename... Args>
-static void launch_chained(void (*kernel)(Params...), int grid, int threads, cudaStream_t st, Args... args) {
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)grid);
-    cfg.blockDim = dim3((unsigned)threads);
-    cfg.stream = st;
-    cudaLaunchAttribute at = {};
-    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at.val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = &at;
-    cfg.numAttrs = 1;
-    cudaLaunchKernelEx(&cfg, kernel, static_cast<Params>(args)...);
-}
 
 void launch_mlp_grad(const float *params, const uint32_t *pack, const float *features, const float *esj, long long n,
                      int n_eps, const float *eps_grid_dev, float eps_min, float eps_max, float *partial, float *grad,

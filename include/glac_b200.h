@@ -87,7 +87,8 @@ uint64_t glac_launch_count(const glac_ctx *ctx);
  *   per plane instead of the ten of a separate clover pass), and the last one
  *   in a pass of its own; 1 uses the compiler's register allocation (FP64: at
  *   three blocks per SM), 2 a 128-register variant, and in FP32 3 a thread per
- *   site and 4 a 96-register variant; 0 measures every field in a pass of its own.  The
+ *   site and 4 a 96-register variant (at the default, small lattices use a
+ *   kernel with several warps to a link); 0 measures every field in a pass of its own.  The
  *   results are the same to rounding.
  *   "fused_combine" (default 1): with fused_measure on, the measurement's
  *   per-site combination and block reduction run inside the step's second
@@ -157,7 +158,9 @@ glac_status glac_flow_configuration(glac_ctx *ctx, const double *host_links, int
 glac_status glac_flow_stage_times(glac_ctx *ctx, int n_steps, double *seconds3);
 /* The same for flow steps that measure the field before each step inside
  * stage 0 ("fused_measure" on): seconds4 = [stage 0 with the clover parts,
- * the measurement's per-site combination and reduction, stage 1, stage 2].
+ * the measurement's per-site combination where that is a pass of its own,
+ * stage 1, stage 2]; the final sum over blocks, made once for many steps of a
+ * flow, is not in it.
  * GLAC_ERR_STATE where the measurement is not fused for this context. */
 glac_status glac_flow_stage_times_measured(glac_ctx *ctx, int n_steps, double *seconds4);
 

@@ -211,6 +211,31 @@ def test_flow_variants_agree(g, oracle, prec):
 
 
 @pytest.mark.parametrize("prec", ["fp64", "fp32"])
+@pytest.mark.parametrize("N", [(4, 4, 4, 4), (4, 6, 6, 6), (10, 6, 4, 6), (8, 8, 4, 16), (8, 8, 16, 18), (16, 16, 16, 10),
+                               (16, 16, 16, 12)])
+def test_small_lattice_flow_matches_oracle(g, oracle, prec, N):
+    # the kernel that gives each link of a small lattice several warps: half
+    # slices that are and are not whole 32-site blocks, planes with a ragged last
+    # block, and the sizes on both sides of where it ends (FP64 18,944 sites, FP32
+    # 42,624); against the oracle and against a thread per link (variant 1)
+    with lattice(g, N, "fp64", beta=6.0, seed=5) as C:
+        C.set_links(oracle.haar_field(N, 5))
+        C.metropolis(10)
+        start = C.get_links()
+    with lattice(g, N, prec) as A, lattice(g, N, prec) as B:
+        B.tuning = [1, 0, 0]
+        A.set_links(start)
+        B.set_links(start)
+        oa, ob = A.flow(2), B.flow(2)
+        want = oracle.flow(N, start, 0.01, 1)
+        assert_obs_close(oa[0], oracle.observables(N, start), TOL[prec], "t = 0")
+        assert_obs_close(oa[1], oracle.observables(N, want), 2 * TOL[prec], "after one step")
+        assert_obs_close(oa, ob, 2 * TOL[prec], "variant 1")
+        assert rel_err(A.get_links(), oracle.flow(N, want, 0.01, 1)) < 2 * TOL[prec]
+        assert rel_err(A.get_links(), B.get_links()) < 2 * TOL[prec]
+
+
+@pytest.mark.parametrize("prec", ["fp64", "fp32"])
 @pytest.mark.parametrize("N", [(6, 4, 6, 8), (8, 8, 8, 16)])
 def test_measurement_inside_flow_stage0(g, oracle, prec, N):
     # glac_flow measures the field before each step inside that step's stage 0
