@@ -64,7 +64,7 @@ void ck_launch(const char *what) { ck(cudaGetLastError(), what); }
 size_t field_bytes(const glac_desc &d, const Geom &g) {
     const size_t vh32 = (size_t)round32(g.Vh);
     if (d.precision == GLAC_FP64) return 8 * vh32 * 9 * sizeof(double2);
-    return 8 * vh32 * 4 * sizeof(float4) + 8 * (size_t)g.Vh * sizeof(float2);
+    return 8 * vh32 * 4 * sizeof(float4) + 8 * vh32 * sizeof(float2);
 }
 size_t force_bytes(const glac_desc &d, const Geom &g) {
     const size_t vh32 = (size_t)round32(g.Vh);
@@ -128,15 +128,6 @@ void ensure_obs(glac_ctx *c, size_t n) {
     c->obs_cap = n;
 }
 
-void measure_into(glac_ctx *c, double *dev_out) {
-    if (c->d.precision == GLAC_FP64)
-        launch_observables(c->g, f64(c, c->cur), c->plan, c->partial, dev_out, c->tune[FAM_OBS], c->stream);
-    else
-        launch_observables(c->g, f32(c, c->cur), c->plan, c->partial, dev_out, c->tune[FAM_OBS], c->stream);
-    ck_launch("observables");
-    c->launches += 2;
-}
-
 // Clover parts: 12 slots of 8-real matrices per site (ForceField layout with a
 // slot index for the direction) followed by the 4 plaquette sums per site.
 size_t clover_ah_bytes(const glac_desc &d, const Geom &g) { return 3 * force_bytes(d, g); }
@@ -191,15 +182,6 @@ FlowMode flow_mode(const glac_ctx *c) {
     m.row = (size_t)6 * m.nb * c->g.N[3];
     return m;
 }
-void ensure_flow_partial(glac_ctx *c, size_t n) {
-    if (c->flow_partial_cap >= n) return;
-    if (c->flow_partial) cudaFree(c->flow_partial);
-    c->flow_partial = nullptr;
-    c->flow_partial_cap = 0;
-    ck(cudaMalloc(&c->flow_partial, n * sizeof(double)), "cudaMalloc flow partials");
-    c->flow_partial_cap = n;
-}
-
 template <typename T> LinkField<T> link_field(glac_ctx *c, int i) {
     if constexpr (sizeof(T) == 8) return f64(c, i);
     else return f32(c, i);
@@ -207,6 +189,38 @@ template <typename T> LinkField<T> link_field(glac_ctx *c, int i) {
 template <typename T> ForceField<T> force_field(glac_ctx *c) {
     if constexpr (sizeof(T) == 8) return z64(c);
     else return z32(c);
+}
+// The stand-alone measurement's parts: slots 0-8 in the field that is not
+// current, the others and the plaquettes in the force (neither holds anything
+// between flow steps).
+template <typename T> PlaneParts<T> plane_parts(glac_ctx *c) {
+    PlaneParts<T> v;
+    v.lo.p = reinterpret_cast<decltype(v.lo.p)>(c->field[c->cur ^ 1]);
+    v.hi.p = reinterpret_cast<decltype(v.hi.p)>(c->force);
+    v.lo.Vh = v.hi.Vh = c->g.Vh;
+    v.lo.Vh32 = v.hi.Vh32 = round32(c->g.Vh);
+    v.plaq = reinterpret_cast<T *>(static_cast<char *>(c->force) + force_bytes(c->d, c->g) / 4 * 3);
+    return v;
+}
+
+void measure_into(glac_ctx *c, double *dev_out) {
+    if (c->d.precision == GLAC_FP64)
+        launch_observables(c->g, f64(c, c->cur), plane_parts<double>(c), c->plan, c->partial, dev_out,
+                           c->tune[FAM_OBS], c->stream);
+    else
+        launch_observables(c->g, f32(c, c->cur), plane_parts<float>(c), c->plan, c->partial, dev_out,
+                           c->tune[FAM_OBS], c->stream);
+    ck_launch("observables");
+    c->launches += 3;
+}
+
+void ensure_flow_partial(glac_ctx *c, size_t n) {
+    if (c->flow_partial_cap >= n) return;
+    if (c->flow_partial) cudaFree(c->flow_partial);
+    c->flow_partial = nullptr;
+    c->flow_partial_cap = 0;
+    ck(cudaMalloc(&c->flow_partial, n * sizeof(double)), "cudaMalloc flow partials");
+    c->flow_partial_cap = n;
 }
 
 // One Luscher RK3 step: three fused stages, cur -> other -> cur -> other.
@@ -584,11 +598,11 @@ glac_status glac_measure_density(glac_ctx *c, double *obs, double *q_density, do
         ensure_staging(c);  // V * 72 doubles: room for both densities
         double *dq = c->staging, *de = c->staging + V;
         if (c->d.precision == GLAC_FP64)
-            launch_observables_density(c->g, f64(c, c->cur), c->plan, c->partial, c->obs_dev, dq, de, c->stream);
+            launch_observables_density(c->g, f64(c, c->cur), plane_parts<double>(c), c->plan, c->partial, c->obs_dev, dq, de, c->stream);
         else
-            launch_observables_density(c->g, f32(c, c->cur), c->plan, c->partial, c->obs_dev, dq, de, c->stream);
+            launch_observables_density(c->g, f32(c, c->cur), plane_parts<float>(c), c->plan, c->partial, c->obs_dev, dq, de, c->stream);
         ck_launch("observables density");
-        c->launches += 2;
+        c->launches += 3;
         if (obs) ck(cudaMemcpyAsync(obs, c->obs_dev, n * sizeof(double), cudaMemcpyDeviceToHost, c->stream), "D2H");
         ck(cudaMemcpyAsync(q_density, dq, V * sizeof(double), cudaMemcpyDeviceToHost, c->stream), "D2H q");
         ck(cudaMemcpyAsync(e_density, de, V * sizeof(double), cudaMemcpyDeviceToHost, c->stream), "D2H e");
@@ -608,10 +622,12 @@ glac_status glac_measure_weinberg(glac_ctx *c, double *obs) {
         const size_t n = 4 + 2 * (size_t)c->g.N[3];
         ensure_obs(c, n);
         if (!c->partial4) ck(cudaMalloc(&c->partial4, 4 * (size_t)c->plan.nblocks * sizeof(double)), "partials");
-        if (c->d.precision == GLAC_FP64) launch_weinberg(c->g, f64(c, c->cur), c->plan, c->partial4, c->obs_dev, c->stream);
-        else launch_weinberg(c->g, f32(c, c->cur), c->plan, c->partial4, c->obs_dev, c->stream);
+        if (c->d.precision == GLAC_FP64)
+            launch_weinberg(c->g, f64(c, c->cur), plane_parts<double>(c), c->plan, c->partial4, c->obs_dev, c->stream);
+        else
+            launch_weinberg(c->g, f32(c, c->cur), plane_parts<float>(c), c->plan, c->partial4, c->obs_dev, c->stream);
         ck_launch("weinberg");
-        c->launches += 2;
+        c->launches += 3;
         ck(cudaMemcpyAsync(obs, c->obs_dev, n * sizeof(double), cudaMemcpyDeviceToHost, c->stream), "D2H");
         ck(cudaStreamSynchronize(c->stream), "sync");
         return GLAC_OK;

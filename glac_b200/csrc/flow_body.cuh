@@ -98,6 +98,14 @@ __device__ __forceinline__ double warp_sum_d(double v) {
     return v;
 }
 
+// en += sum ReTr(F F) and qt = -[ReTr(F_01 F_23) + ReTr(F_02 F_31) + ReTr(F_03 F_12)]
+// (F_31 = -F_13) of a site's six projected clovers.
+template <typename T> __device__ __forceinline__ void clover_sums(const AH8<T> F[6], double &en, double &qt) {
+    qt = -((double)retr_ah(F[0], F[5]) - (double)retr_ah(F[1], F[4]) + (double)retr_ah(F[2], F[3]));
+#pragma unroll
+    for (int pl = 0; pl < 6; pl++) en += (double)retr_ah(F[pl], F[pl]);
+}
+
 template <typename T>
 __device__ __forceinline__ void combine_site(const Geom &g, const CloverParts<T> &cp, int p, int s, double &plaq,
                                              double &en, double &qt) {
@@ -106,10 +114,62 @@ __device__ __forceinline__ void combine_site(const Geom &g, const CloverParts<T>
     for (int pl = 0; pl < 6; pl++) F[pl] = ah_add(cp.ah.load(2 * pl, p, s), cp.ah.load(2 * pl + 1, p, s));
 #pragma unroll
     for (int mu = 0; mu < 4; mu++) plaq += (double)cp.plaq[(mu * 2 + p) * g.Vh + s];
-    // q = -[ReTr(F_01 F_23) + ReTr(F_02 F_31) + ReTr(F_03 F_12)], F_31 = -F_13
-    qt = -((double)retr_ah(F[0], F[5]) - (double)retr_ah(F[1], F[4]) + (double)retr_ah(F[2], F[3]));
-#pragma unroll
-    for (int pl = 0; pl < 6; pl++) en += (double)retr_ah(F[pl], F[pl]);
+    clover_sums(F, en, qt);
 }
 
+// Block sums of the three per-thread values in a fixed order (warp shuffles,
+// then the warps in order) into partial[3 b .. 3 b + 2] = (plaq, energy, q).
+__device__ __forceinline__ void obs_block_reduce(double plaq, double en, double qt, double *partial, int b) {
+    __shared__ double sh[3][32];
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    plaq = warp_sum_d(plaq);
+    en = warp_sum_d(en);
+    qt = warp_sum_d(qt);
+    if (lane == 0) { sh[0][wid] = plaq; sh[1][wid] = en; sh[2][wid] = qt; }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        const int nw = (blockDim.x + 31) >> 5;
+        double a = 0.0, e = 0.0, q = 0.0;
+        for (int w = 0; w < nw; w++) { a += sh[0][w]; e += sh[1][w]; q += sh[2][w]; }
+        partial[3 * b] = a;
+        partial[3 * b + 1] = e;
+        partial[3 * b + 2] = q;
+    }
+}
+
+// out = [plaq, topc, energy, topct[Nt]] with the reference's normalisations
+// (mastersamplertopcxyz.cpp:13-16, :363-383).
+// Per-slice sums by warps (slice t on warp t mod W; lane l adds the partials
+// l, l+32, ..., then a fixed xor-shuffle tree), the slices then in order by one
+// thread: the same operations in the same order every call.
+__device__ __forceinline__ void obs_finalize_body(int Nt, int nb, int V, const double *partial, double *out) {
+    __shared__ double sp[1024], se[1024], sq[1024];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
+    for (int t = warp; t < Nt; t += nwarps) {
+        double a = 0.0, e = 0.0, q = 0.0;
+        const double *pt = partial + 3 * (size_t)t * 2 * nb;
+        for (int k = lane; k < 2 * nb; k += 32) {
+            a += pt[3 * k];
+            e += pt[3 * k + 1];
+            q += pt[3 * k + 2];
+        }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            a += __shfl_xor_sync(0xffffffffu, a, o);
+            e += __shfl_xor_sync(0xffffffffu, e, o);
+            q += __shfl_xor_sync(0xffffffffu, q, o);
+        }
+        if (lane == 0) { sp[t] = a; se[t] = e; sq[t] = q; }
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        const double qfac = 1.0 / (16 * 16 * M_PI * M_PI);
+        double a = 0.0, e = 0.0, q = 0.0;
+        for (int t = 0; t < Nt; t++) { a += sp[t]; e += se[t]; q += sq[t]; }
+        out[0] = a / (18.0 * (double)V);
+        out[1] = q * qfac;
+        out[2] = e / (double)V;
+        for (int t = 0; t < Nt; t++) out[3 + t] = sq[t] * qfac;
+    }
+}
 }  // namespace glac

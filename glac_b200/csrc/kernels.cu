@@ -915,33 +915,9 @@ __device__ __forceinline__ AH8<T> clover_ah(const LinkField<T> &L, const Geom &g
     else return clover_ah_call<T>(L, g, n, p, mu, nu, plaq);
 }
 
-// Block sums of the three per-thread values in a fixed order (warp shuffles,
-// then the warps in order) into partial[3 b .. 3 b + 2] = (plaq, energy, q).
-__device__ __forceinline__ void obs_block_reduce(double plaq, double en, double qt, double *partial, int b) {
-    __shared__ double sh[3][32];
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    plaq = warp_sum_d(plaq);
-    en = warp_sum_d(en);
-    qt = warp_sum_d(qt);
-    if (lane == 0) { sh[0][wid] = plaq; sh[1][wid] = en; sh[2][wid] = qt; }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        const int nw = (blockDim.x + 31) >> 5;
-        double a = 0.0, e = 0.0, q = 0.0;
-        for (int w = 0; w < nw; w++) { a += sh[0][w]; e += sh[1][w]; q += sh[2][w]; }
-        partial[3 * b] = a;
-        partial[3 * b + 1] = e;
-        partial[3 * b + 2] = q;
-    }
-}
-
-// With dq/de set, also the per-site densities in lexicographic order:
-// dq[n] = -(1/(16^2 pi^2)) sum ReTr(C_0nu C_rhosigma), de[n] = sum ReTr(C C) (unnormalised),
-// the fields LatticeActionChargeDensity writes (latticeactionchargedensity.cpp:169-306).
 template <typename T>
 __device__ __forceinline__ void observables_body(const Geom &g, const LinkField<T> &L, int nb, int Bv,
-                                                 double *partial, int b, double *dq = nullptr,
-                                                 double *de = nullptr) {
+                                                 double *partial, int b) {
     const int t = b / (2 * nb);
     const int p = (b / nb) & 1;
     const int j = b % nb;
@@ -962,86 +938,10 @@ __device__ __forceinline__ void observables_body(const Geom &g, const LinkField<
             qt -= (double)retr_ah(F1, F2);
             en += (double)retr_ah(F1, F1) + (double)retr_ah(F2, F2);
         }
-        if (dq) {
-            dq[n.lex] = qt * (1.0 / (16 * 16 * M_PI * M_PI));
-            de[n.lex] = en;
-        }
     }
     obs_block_reduce(plaq, en, qt, partial, b);
 }
 
-#define GLAC_OBS_KERNEL(NAME, ATTR)                                                                      \
-    template <typename T>                                                                              \
-    __global__ void ATTR NAME(Geom g, LinkField<T> L, int nb, int Bv, double *partial) {               \
-        observables_body<T>(g, L, nb, Bv, partial, blockIdx.x);                                        \
-    }
-GLAC_OBS_KERNEL(k_observables, __launch_bounds__(256))
-GLAC_OBS_KERNEL(k_observables_r168, __maxnreg__(168))
-GLAC_OBS_KERNEL(k_observables_r128, __maxnreg__(128))
-GLAC_OBS_KERNEL(k_observables_r96, __maxnreg__(96))
-#undef GLAC_OBS_KERNEL
-
-// out = [plaq, topc, energy, topct[Nt]] with the reference's normalisations
-// (mastersamplertopcxyz.cpp:13-16, :363-383).
-// Per-slice sums by warps (slice t on warp t mod W; lane l adds the partials
-// l, l+32, ..., then a fixed xor-shuffle tree), the slices then in order by one
-// thread: the same operations in the same order every call.
-__device__ __forceinline__ void obs_finalize_body(int Nt, int nb, int V, const double *partial, double *out) {
-    __shared__ double sp[1024], se[1024], sq[1024];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
-    for (int t = warp; t < Nt; t += nwarps) {
-        double a = 0.0, e = 0.0, q = 0.0;
-        const double *pt = partial + 3 * (size_t)t * 2 * nb;
-        for (int k = lane; k < 2 * nb; k += 32) {
-            a += pt[3 * k];
-            e += pt[3 * k + 1];
-            q += pt[3 * k + 2];
-        }
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-            a += __shfl_xor_sync(0xffffffffu, a, o);
-            e += __shfl_xor_sync(0xffffffffu, e, o);
-            q += __shfl_xor_sync(0xffffffffu, q, o);
-        }
-        if (lane == 0) { sp[t] = a; se[t] = e; sq[t] = q; }
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        const double qfac = 1.0 / (16 * 16 * M_PI * M_PI);
-        double a = 0.0, e = 0.0, q = 0.0;
-        for (int t = 0; t < Nt; t++) { a += sp[t]; e += se[t]; q += sq[t]; }
-        out[0] = a / (18.0 * (double)V);
-        out[1] = q * qfac;
-        out[2] = e / (double)V;
-        for (int t = 0; t < Nt; t++) out[3 + t] = sq[t] * qfac;
-    }
-}
-// One measurement per block: rows of 3 (2 nb Nt) partials in, rows of 3 + Nt out.
-__global__ void k_obs_finalize(int Nt, int nb, int V, const double *partial, double *out) {
-    obs_finalize_body(Nt, nb, V, partial + (size_t)blockIdx.x * 6 * nb * Nt, out + (size_t)blockIdx.x * (3 + Nt));
-}
-void launch_obs_finalize(const Geom &g, int nb, int rows, const double *partial, double *out, cudaStream_t st) {
-    if (g.N[3] > 1024) throw std::invalid_argument("Nt > 1024 not supported by the observable reduction");
-    k_obs_finalize<<<rows, 1024, 0, st>>>(g.N[3], nb, g.V, partial, out);
-}
-
-template <typename T>
-void launch_observables(const Geom &g, const LinkField<T> &L, const ObsPlan &plan, double *partial, double *out,
-                        int variant, cudaStream_t st) {
-    if (g.N[3] > 1024) throw std::invalid_argument("Nt > 1024 not supported by the observable reduction");
-    switch (variant_regs(FAM_OBS, sizeof(T) == 4, variant)) {
-    case 168:
-        if constexpr (sizeof(T) == 4) {
-            k_observables_r168<T><<<plan.nblocks, plan.B, 0, st>>>(g, L, plan.nb, plan.Bv, partial);
-            break;
-        }
-        [[fallthrough]];
-    case 128: k_observables_r128<T><<<plan.nblocks, plan.B, 0, st>>>(g, L, plan.nb, plan.Bv, partial); break;
-    case 96: k_observables_r96<T><<<plan.nblocks, plan.B, 0, st>>>(g, L, plan.nb, plan.Bv, partial); break;
-    default: k_observables<T><<<plan.nblocks, plan.B, 0, st>>>(g, L, plan.nb, plan.Bv, partial); break;
-    }
-    k_obs_finalize<<<1, 1024, 0, st>>>(g.N[3], plan.nb, g.V, partial, out);
-}
 // The measurement from the parts that flow stage 0 wrote (flow_stage0_meas_body):
 // per site F of each plane = its local + forward slot, the plaquette = the four
 // direction sums; Q(t), E and the plaquette reduced as in observables_body (same
@@ -1159,148 +1059,6 @@ template void launch_obs_combine<double>(const Geom &, const CloverParts<double>
                                          cudaStream_t);
 template void launch_obs_combine<float>(const Geom &, const CloverParts<float> &, const ObsPlan &, double *,
                                         cudaStream_t);
-
-template <typename T>
-__global__ void __launch_bounds__(256) k_observables_density(Geom g, LinkField<T> L, int nb, int Bv, double *partial,
-                                                             double *dq, double *de) {
-    observables_body<T>(g, L, nb, Bv, partial, blockIdx.x, dq, de);
-}
-template <typename T>
-void launch_observables_density(const Geom &g, const LinkField<T> &L, const ObsPlan &plan, double *partial,
-                                double *out, double *dq, double *de, cudaStream_t st) {
-    if (g.N[3] > 1024) throw std::invalid_argument("Nt > 1024 not supported by the observable reduction");
-    k_observables_density<T><<<plan.nblocks, plan.B, 0, st>>>(g, L, plan.nb, plan.Bv, partial, dq, de);
-    k_obs_finalize<<<1, 1024, 0, st>>>(g.N[3], plan.nb, g.V, partial, out);
-}
-template void launch_observables_density<double>(const Geom &, const LinkField<double> &, const ObsPlan &, double *,
-                                                 double *, double *, double *, cudaStream_t);
-template void launch_observables_density<float>(const Geom &, const LinkField<float> &, const ObsPlan &, double *,
-                                                double *, double *, double *, cudaStream_t);
-template void launch_observables<double>(const Geom &, const LinkField<double> &, const ObsPlan &, double *,
-                                         double *, int, cudaStream_t);
-template void launch_observables<float>(const Geom &, const LinkField<float> &, const ObsPlan &, double *,
-                                        double *, int, cudaStream_t);
-
-// ---------------------------------------------------------------------------
-// SuperSampler (GLAC/observables/supersampler.cpp:298-496): the observables
-// above plus the Weinberg operator.  With the six projected clovers G of a
-// site, for nu = 1..3 and (rho, sigma) the cyclic complement of nu:
-//   w(t) -= ReTr[(sum_{lambda != nu} G_{0 lambda} G_{nu lambda}) G_{rho sigma}],
-// factor 2 * 8 * 8 / (3 * 16^3) (:13).  G_{b a} = G_{a b}^+ for the
-// orientations the reference does not store (:421-433).  Partials: 4 per block.
-// ---------------------------------------------------------------------------
-template <typename T>
-__global__ void __launch_bounds__(256) k_observables_weinberg(Geom g, LinkField<T> L, int nb, int Bv,
-                                                              double *partial) {
-    const int b = blockIdx.x;
-    const int t = b / (2 * nb);
-    const int p = (b / nb) & 1;
-    const int j = b % nb;
-    const int half_slice = g.Vh / g.N[3];
-    const bool valid = (int)threadIdx.x < Bv;
-    const int s = t * half_slice + j * Bv + (valid ? (int)threadIdx.x : 0);
-    double plaq = 0.0, en = 0.0, qt = 0.0, wt = 0.0;
-    if (valid) {
-        const Site n = site_from_ps(g, p, s);
-        AH8<T> G0[4], Gc[4];  // G0[nu] = G_{0 nu}; Gc[nu] = G_{rho sigma} of nu's complement
-#pragma unroll 1
-        for (int nu = 1; nu < 4; nu++) {
-            const int rho = nu % 3 + 1, sigma = rho % 3 + 1;
-            T pl1, pl2;
-            G0[nu] = clover_ah(L, g, n, p, 0, nu, pl1);
-            Gc[nu] = clover_ah(L, g, n, p, rho, sigma, pl2);
-            plaq += (double)pl1 + (double)pl2;
-            qt -= (double)retr_ah(G0[nu], Gc[nu]);
-            en += (double)retr_ah(G0[nu], G0[nu]) + (double)retr_ah(Gc[nu], Gc[nu]);
-        }
-        // G_{a b} for spatial a != b from the stored G_{23} = Gc[1], G_{31} = Gc[2], G_{12} = Gc[3]
-        auto spatial = [&](int a, int c) -> M3<T> {
-            // (a, c) in {(1,2),(2,3),(3,1)} is stored as Gc[the third index]; the reverse is its dagger
-            const int k = 6 - a - c;
-            const bool stored = (c == a % 3 + 1);
-            const M3<T> m = ah_to_m3(Gc[k]);
-            return stored ? m : dagger(m);
-        };
-#pragma unroll 1
-        for (int nu = 1; nu < 4; nu++) {
-            M3<T> acc;
-            set_zero(acc);
-#pragma unroll 1
-            for (int lam = 1; lam < 4; lam++) {
-                if (lam == nu) continue;
-                acc_mul(acc, ah_to_m3(G0[lam]), spatial(nu, lam));
-            }
-            wt -= (double)retr_mul(acc, ah_to_m3(Gc[nu]));
-        }
-    }
-    __shared__ double sh[4][32];
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    plaq = warp_sum_d(plaq);
-    en = warp_sum_d(en);
-    qt = warp_sum_d(qt);
-    wt = warp_sum_d(wt);
-    if (lane == 0) { sh[0][wid] = plaq; sh[1][wid] = en; sh[2][wid] = qt; sh[3][wid] = wt; }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        const int nw = (blockDim.x + 31) >> 5;
-        double a = 0.0, e = 0.0, q = 0.0, w = 0.0;
-        for (int k = 0; k < nw; k++) { a += sh[0][k]; e += sh[1][k]; q += sh[2][k]; w += sh[3][k]; }
-        partial[4 * b] = a;
-        partial[4 * b + 1] = e;
-        partial[4 * b + 2] = q;
-        partial[4 * b + 3] = w;
-    }
-}
-
-// out = [plaq, topc, energy, weinberg, topct[Nt], weinbergt[Nt]]
-__global__ void k_weinberg_finalize(int Nt, int nb, int V, const double *partial, double *out) {
-    __shared__ double sp[1024], se[1024], sq[1024], sw[1024];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
-    for (int t = warp; t < Nt; t += nwarps) {
-        double a = 0.0, e = 0.0, q = 0.0, w = 0.0;
-        const double *pt = partial + 4 * (size_t)t * 2 * nb;
-        for (int k = lane; k < 2 * nb; k += 32) {
-            a += pt[4 * k];
-            e += pt[4 * k + 1];
-            q += pt[4 * k + 2];
-            w += pt[4 * k + 3];
-        }
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-            a += __shfl_xor_sync(0xffffffffu, a, o);
-            e += __shfl_xor_sync(0xffffffffu, e, o);
-            q += __shfl_xor_sync(0xffffffffu, q, o);
-            w += __shfl_xor_sync(0xffffffffu, w, o);
-        }
-        if (lane == 0) { sp[t] = a; se[t] = e; sq[t] = q; sw[t] = w; }
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        const double qfac = 1.0 / (16 * 16 * M_PI * M_PI), wfac = 2 * 8.0 * 8.0 / (3 * 16 * 16 * 16);
-        double a = 0.0, e = 0.0, q = 0.0, w = 0.0;
-        for (int t = 0; t < Nt; t++) { a += sp[t]; e += se[t]; q += sq[t]; w += sw[t]; }
-        out[0] = a / (18.0 * (double)V);
-        out[1] = q * qfac;
-        out[2] = e / (double)V;
-        out[3] = w * wfac;
-        for (int t = 0; t < Nt; t++) {
-            out[4 + t] = sq[t] * qfac;
-            out[4 + Nt + t] = sw[t] * wfac;
-        }
-    }
-}
-
-template <typename T>
-void launch_weinberg(const Geom &g, const LinkField<T> &L, const ObsPlan &plan, double *partial4, double *out,
-                     cudaStream_t st) {
-    if (g.N[3] > 1024) throw std::invalid_argument("Nt > 1024 not supported by the observable reduction");
-    k_observables_weinberg<T><<<plan.nblocks, plan.B, 0, st>>>(g, L, plan.nb, plan.Bv, partial4);
-    k_weinberg_finalize<<<1, 1024, 0, st>>>(g.N[3], plan.nb, g.V, partial4, out);
-}
-template void launch_weinberg<double>(const Geom &, const LinkField<double> &, const ObsPlan &, double *, double *,
-                                      cudaStream_t);
-template void launch_weinberg<float>(const Geom &, const LinkField<float> &, const ObsPlan &, double *, double *,
-                                     cudaStream_t);
 
 // ---------------------------------------------------------------------------
 // Start fields, reunitarisation, layout conversion

@@ -140,17 +140,18 @@ template <typename T>
 void launch_esj(const Geom &g, const LinkField<T> &L, double beta, int nhits, int n_eps, const float *eps_grid_dev,
                 int trials, int stride, int offset, int ns, uint64_t seed, uint32_t snapshot, uint32_t stream_id,
                 bool flips, float *feat, float *esj, uint32_t *ids, cudaStream_t st);
-// SuperSampler observables: [plaq, topc, energy, weinberg, topct[Nt], weinbergt[Nt]]; partial4: 4 per block.
+// The stand-alone measurement (observables.cu): [plaq, topc, energy, topct[Nt]],
+// the same with per-site densities (V doubles each, lexicographic), and the
+// SuperSampler's [plaq, topc, energy, weinberg, topct[Nt], weinbergt[Nt]] (partial4: 4 per block).
 template <typename T>
-void launch_weinberg(const Geom &g, const LinkField<T> &L, const ObsPlan &plan, double *partial4, double *out,
-                     cudaStream_t st);
-// Observables plus per-site topological-charge and energy densities (V doubles each, lexicographic).
+void launch_observables(const Geom &g, const LinkField<T> &L, const PlaneParts<T> &parts, const ObsPlan &plan,
+                        double *partial, double *out, int variant, cudaStream_t st);
 template <typename T>
-void launch_observables_density(const Geom &g, const LinkField<T> &L, const ObsPlan &plan, double *partial,
-                                double *out, double *dq, double *de, cudaStream_t st);
+void launch_observables_density(const Geom &g, const LinkField<T> &L, const PlaneParts<T> &parts, const ObsPlan &plan,
+                                double *partial, double *out, double *dq, double *de, cudaStream_t st);
 template <typename T>
-void launch_observables(const Geom &g, const LinkField<T> &L, const ObsPlan &plan, double *partial,
-                        double *out, int variant, cudaStream_t st);
+void launch_weinberg(const Geom &g, const LinkField<T> &L, const PlaneParts<T> &parts, const ObsPlan &plan,
+                     double *partial4, double *out, cudaStream_t st);
 template <typename T>
 void launch_haar(const Geom &g, const LinkField<T> &L, uint64_t seed, uint32_t stream_id, cudaStream_t st);
 template <typename T>

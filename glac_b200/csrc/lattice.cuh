@@ -278,6 +278,22 @@ template <typename T> struct CloverParts {
     T *plaq;
 };
 
+// The same twelve slots for the stand-alone measurement, in two buffers: slots
+// 0-8 in one the size of a link field, 9-11 and six plaquettes per site,
+// plaq[(plane * 2 + parity) * Vh + s], in one the size of a force (9 x 8 reals are
+// 4 x 18, and 3 x 8 + 6 fewer than 4 x 8).
+template <typename T> struct PlaneParts {
+    ForceField<T> lo, hi;
+    T *plaq;
+    __device__ __forceinline__ AH8<T> load(int k, int par, int s) const {
+        return k < 9 ? lo.load(k, par, s) : hi.load(k - 9, par, s);
+    }
+    __device__ __forceinline__ void store(int k, int par, int s, const AH8<T> &Z) const {
+        if (k < 9) lo.store(k, par, s, Z);
+        else hi.store(k - 9, par, s, Z);
+    }
+};
+
 // ---------------------------------------------------------------------------
 // Philox4x32-10 (Salmon, Moraes, Dror, Shaw, SC'11)
 // ---------------------------------------------------------------------------
