@@ -225,10 +225,10 @@ GLAC_FLOW_KERNEL(k_flow_stage_r96, __maxnreg__(96))
 // neighbour links (L2 hits), so resident warps count for more than registers:
 // its default caps give 16 (FP64) and 24 (FP32) warps per SM.  Stage 2 on B200,
 // capped / uncapped: FP64 24^3 x 48 427 / 528 us, 16^3 x 32 97 / 114; FP32
-// 32^3 x 64 662 / 700, 16^3 x 32 51 / 53.
+// 32^3 x 64 662 / 700, 16^3 x 32 51 / 53.  Metropolis: see metro_regs.
 const int kFlowRegs[2][kMaxVariants] = {{128, 0, 0, 128}, {80, 0, 0, 96}};
 const int kFlowShape[2][kMaxVariants] = {{0, 0, 1, 2}, {0, 0, 3, 0}};
-const int kMetroRegs[2][kMaxVariants] = {{0, 128, -1, -1}, {0, 96, 80, 128}};
+const int kMetroRegs[2][kMaxVariants] = {{0, 128, -1, -1}, {96, 0, 80, 128}};
 const int kObsRegs[2][kMaxVariants] = {{0, 128, -1, -1}, {0, 128, 168, -1}};
 
 int num_variants(Family f, bool fp32) {
@@ -707,6 +707,16 @@ static void metro_dispatch(int regs, dim3 grid, cudaStream_t st, const Geom &g, 
     }
 }
 
+// Register cap of a sub-sweep.  FP32's default is 96 (five blocks per SM), but
+// 128 (four) where a fifth block finds no work, up to one wave of blocks, and for
+// the learned spread, whose kernel spills at 96.  Microseconds per sweep on B200
+// at 128 / 96: 8^3 x 16 82 / 86, 24^3 x 48 788 / 778, 32^3 x 64 2276 / 2248;
+// learned 24^3 x 48 898 / 934 (uncapped 930).
+static int metro_regs(bool fp32, int variant, bool learned, int blocks) {
+    if (fp32 && variant == 0 && (learned || blocks <= 5 * 148)) return 128;
+    return variant_regs(FAM_METRO, fp32, variant);
+}
+
 template <typename T>
 void launch_metropolis(const Geom &g, const LinkField<T> &L, int mu, int p, double beta, double eps, int nhits,
                        uint64_t seed, uint32_t sweep, uint32_t stream_id, unsigned long long *acc, int variant,
@@ -714,7 +724,7 @@ void launch_metropolis(const Geom &g, const LinkField<T> &L, int mu, int p, doub
     const dim3 grid((g.Vh + 127) / 128);  // 128 threads: the learned path's shared memory holds 4 warps
     const T mfac = (T)(-beta / 3.0), e = (T)eps, sq = (T)sqrt(1.0 - eps * eps);
     const uint32_t k0 = (uint32_t)seed, k1 = (uint32_t)(seed >> 32);
-    const int regs = variant_regs(FAM_METRO, sizeof(T) == 4, variant);
+    const int regs = metro_regs(sizeof(T) == 4, variant, P.net != nullptr, (int)grid.x);
     if (P.net)
         metro_dispatch<T, true>(regs, grid, st, g, L, mu, p, mfac, e, sq, nhits, k0, k1, sweep, stream_id, acc, P,
                                 (float)beta);

@@ -11,6 +11,7 @@
 // hold nothing between flow steps.
 #include "kernels.cuh"
 #include "flow_body.cuh"
+#include "launch.cuh"
 
 #include <stdexcept>
 
@@ -33,12 +34,14 @@ __device__ __forceinline__ void clover_parts_body(const Geom &g, const LinkField
     asm volatile("" ::: "memory");
     sub_mul(W, mul_dd(L.load(nu, p, s_diag), L.load(mu, q, s_num)), L.load(nu, q, s_num));
     asm volatile("" ::: "memory");
+    chain_release();
     parts.store(2 * pl, p, s, clover_part(L.load(mu, p, s), W, false));
     asm volatile("" ::: "memory");
     parts.store(2 * pl + 1, q, s_mu, clover_part(W, L.load(mu, p, s), false));
 }
 template <typename T, int BLOCKS>
 __global__ void __launch_bounds__(128, BLOCKS) k_clover_parts(Geom g, LinkField<T> L, PlaneParts<T> parts) {
+    chain_wait();
     clover_parts_body<T>(g, L, parts, blockIdx.x);
 }
 
@@ -79,6 +82,7 @@ template <typename T> __device__ __forceinline__ double weinberg_site(const AH8<
 template <typename T, ObsMode MODE>
 __global__ void __launch_bounds__(256) k_plane_combine(Geom g, PlaneParts<T> parts, int nb, int Bv, double *partial,
                                                        double *dq, double *de) {
+    chain_wait();
     const int b = blockIdx.x;
     const int t = b / (2 * nb);
     const int p = (b / nb) & 1;
@@ -126,16 +130,18 @@ __global__ void __launch_bounds__(256) k_plane_combine(Geom g, PlaneParts<T> par
 
 // One measurement per block: rows of 3 (2 nb Nt) partials in, rows of 3 + Nt out.
 __global__ void k_obs_finalize(int Nt, int nb, int V, const double *partial, double *out) {
+    chain_wait();
     obs_finalize_body(Nt, nb, V, partial + (size_t)blockIdx.x * 6 * nb * Nt, out + (size_t)blockIdx.x * (3 + Nt));
 }
 void launch_obs_finalize(const Geom &g, int nb, int rows, const double *partial, double *out, cudaStream_t st) {
     if (g.N[3] > 1024) throw std::invalid_argument("Nt > 1024 not supported by the observable reduction");
-    k_obs_finalize<<<rows, 1024, 0, st>>>(g.N[3], nb, g.V, partial, out);
+    launch_chained(k_obs_finalize, rows, 1024, st, g.N[3], nb, g.V, partial, out);
 }
 
 // out = [plaq, topc, energy, weinberg, topct[Nt], weinbergt[Nt]], the Weinberg factor
 // 2 * 8 * 8 / (3 * 16^3) (supersampler.cpp:13)
 __global__ void k_weinberg_finalize(int Nt, int nb, int V, const double *partial, double *out) {
+    chain_wait();
     __shared__ double sp[1024], se[1024], sq[1024], sw[1024];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
     for (int t = warp; t < Nt; t += nwarps) {
@@ -178,12 +184,12 @@ static void clover_parts(const Geom &g, const LinkField<T> &L, const PlaneParts<
     if (g.N[3] > 1024) throw std::invalid_argument("Nt > 1024 not supported by the observable reduction");
     const int grid = 12 * ((g.Vh + 127) / 128);
     if constexpr (sizeof(T) == 4) {
-        if (variant == 1) k_clover_parts<T, 4><<<grid, 128, 0, st>>>(g, L, parts);
-        else if (variant == 2) k_clover_parts<T, 5><<<grid, 128, 0, st>>>(g, L, parts);
-        else k_clover_parts<T, 6><<<grid, 128, 0, st>>>(g, L, parts);
+        if (variant == 1) launch_chained(k_clover_parts<T, 4>, grid, 128, st, g, L, parts);
+        else if (variant == 2) launch_chained(k_clover_parts<T, 5>, grid, 128, st, g, L, parts);
+        else launch_chained(k_clover_parts<T, 6>, grid, 128, st, g, L, parts);
     } else {
-        if (variant == 1) k_clover_parts<T, 3><<<grid, 128, 0, st>>>(g, L, parts);
-        else k_clover_parts<T, 4><<<grid, 128, 0, st>>>(g, L, parts);
+        if (variant == 1) launch_chained(k_clover_parts<T, 3>, grid, 128, st, g, L, parts);
+        else launch_chained(k_clover_parts<T, 4>, grid, 128, st, g, L, parts);
     }
 }
 
@@ -191,23 +197,24 @@ template <typename T>
 void launch_observables(const Geom &g, const LinkField<T> &L, const PlaneParts<T> &parts, const ObsPlan &plan,
                         double *partial, double *out, int variant, cudaStream_t st) {
     clover_parts(g, L, parts, variant, st);
-    k_plane_combine<T, OBS_SUMS><<<plan.nblocks, plan.B, 0, st>>>(g, parts, plan.nb, plan.Bv, partial, nullptr, nullptr);
+    launch_chained(k_plane_combine<T, OBS_SUMS>, plan.nblocks, plan.B, st, g, parts, plan.nb, plan.Bv, partial,
+                   static_cast<double *>(nullptr), static_cast<double *>(nullptr));
     launch_obs_finalize(g, plan.nb, 1, partial, out, st);
 }
 template <typename T>
 void launch_observables_density(const Geom &g, const LinkField<T> &L, const PlaneParts<T> &parts, const ObsPlan &plan,
                                 double *partial, double *out, double *dq, double *de, cudaStream_t st) {
     clover_parts(g, L, parts, 0, st);
-    k_plane_combine<T, OBS_DENSITY><<<plan.nblocks, plan.B, 0, st>>>(g, parts, plan.nb, plan.Bv, partial, dq, de);
+    launch_chained(k_plane_combine<T, OBS_DENSITY>, plan.nblocks, plan.B, st, g, parts, plan.nb, plan.Bv, partial, dq, de);
     launch_obs_finalize(g, plan.nb, 1, partial, out, st);
 }
 template <typename T>
 void launch_weinberg(const Geom &g, const LinkField<T> &L, const PlaneParts<T> &parts, const ObsPlan &plan,
                      double *partial4, double *out, cudaStream_t st) {
     clover_parts(g, L, parts, 0, st);
-    k_plane_combine<T, OBS_WEINBERG><<<plan.nblocks, plan.B, 0, st>>>(g, parts, plan.nb, plan.Bv, partial4, nullptr,
-                                                                     nullptr);
-    k_weinberg_finalize<<<1, 1024, 0, st>>>(g.N[3], plan.nb, g.V, partial4, out);
+    launch_chained(k_plane_combine<T, OBS_WEINBERG>, plan.nblocks, plan.B, st, g, parts, plan.nb, plan.Bv, partial4,
+                   static_cast<double *>(nullptr), static_cast<double *>(nullptr));
+    launch_chained(k_weinberg_finalize, 1, 1024, st, g.N[3], plan.nb, g.V, partial4, out);
 }
 
 #define GLAC_OBS_INST(T)                                                                                             \
