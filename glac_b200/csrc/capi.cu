@@ -1,6 +1,7 @@
 // C ABI (include/glac_b200.h): contexts, device buffers, stream, and the
 // sequencing of the hot-path kernels.
 #include "../../include/glac_b200.h"
+#include "hostcopy.cuh"
 #include "kernels.cuh"
 
 #include <cuda_runtime.h>
@@ -326,6 +327,7 @@ glac_status glac_create(const glac_desc *desc, glac_ctx **out) {
     if (!(d.su3_eps > 0.0 && d.su3_eps < 1.0)) { g_global_err = "su3_eps must lie in (0, 1)"; return GLAC_ERR_ARG; }
     if (d.dims[3] > 1024) { g_global_err = "Nt > 1024 is not supported"; return GLAC_ERR_ARG; }
     glac_ctx *c = new glac_ctx();
+    hostcopy_hold();
     c->d = d;
     c->g = make_geom(d.dims);
     c->plan = make_obs_plan(c->g);
@@ -369,6 +371,7 @@ void glac_destroy(glac_ctx *c) {
     if (c->esj_grid) cudaFree(c->esj_grid);
     if (c->clover) cudaFree(c->clover);
     if (c->stream) cudaStreamDestroy(c->stream);
+    hostcopy_drop();
     delete c;
 }
 
@@ -471,9 +474,7 @@ glac_status glac_set_links(glac_ctx *c, const double *host) {
     return guarded(c, [&] {
         if (!host) { c->err = "null field"; return GLAC_ERR_ARG; }
         ensure_staging(c);
-        ck(cudaMemcpyAsync(c->staging, host, (size_t)c->g.V * 72 * sizeof(double), cudaMemcpyHostToDevice,
-                           c->stream),
-           "H2D links");
+        ck(copy_to_device(c->staging, host, (size_t)c->g.V * 72 * sizeof(double), c->d.device, c->stream), "H2D links");
         glac_status s = glac_set_links_device(c, c->staging);
         if (s != GLAC_OK) return s;
         ck(cudaStreamSynchronize(c->stream), "sync");
@@ -487,10 +488,7 @@ glac_status glac_get_links(glac_ctx *c, double *host) {
         ensure_staging(c);
         glac_status s = glac_get_links_device(c, c->staging);
         if (s != GLAC_OK) return s;
-        ck(cudaMemcpyAsync(host, c->staging, (size_t)c->g.V * 72 * sizeof(double), cudaMemcpyDeviceToHost,
-                           c->stream),
-           "D2H links");
-        ck(cudaStreamSynchronize(c->stream), "sync");
+        ck(copy_to_host(host, c->staging, (size_t)c->g.V * 72 * sizeof(double), c->d.device, c->stream), "D2H links");
         return GLAC_OK;
     });
 }
@@ -604,9 +602,8 @@ glac_status glac_measure_density(glac_ctx *c, double *obs, double *q_density, do
         ck_launch("observables density");
         c->launches += 3;
         if (obs) ck(cudaMemcpyAsync(obs, c->obs_dev, n * sizeof(double), cudaMemcpyDeviceToHost, c->stream), "D2H");
-        ck(cudaMemcpyAsync(q_density, dq, V * sizeof(double), cudaMemcpyDeviceToHost, c->stream), "D2H q");
-        ck(cudaMemcpyAsync(e_density, de, V * sizeof(double), cudaMemcpyDeviceToHost, c->stream), "D2H e");
-        ck(cudaStreamSynchronize(c->stream), "sync");
+        ck(copy_to_host(q_density, dq, V * sizeof(double), c->d.device, c->stream), "D2H q");
+        ck(copy_to_host(e_density, de, V * sizeof(double), c->d.device, c->stream), "D2H e");
         return GLAC_OK;
     });
 }

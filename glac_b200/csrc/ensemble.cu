@@ -13,6 +13,7 @@
 // counter of the Philox streams lives in device memory, so replays draw fresh
 // numbers.
 #include "../../include/glac_b200.h"
+#include "hostcopy.cuh"
 #include "kernels.cuh"
 
 #include <cuda_runtime.h>
@@ -339,6 +340,7 @@ glac_status glac_ensemble_create(int n, const int *dims, const double *betas, co
         }
     }
     glac_ensemble *E = new glac_ensemble;
+    hostcopy_hold();
     E->d = *common;
     E->M = n;
     glac_status s = eguarded(E, [&] {
@@ -405,6 +407,7 @@ void glac_ensemble_destroy(glac_ensemble *E) {
     for (int k = 0; k < ENS_NPHASE; k++)
         if (E->start[k]) cudaFree(E->start[k]);
     if (E->stream) cudaStreamDestroy(E->stream);
+    hostcopy_drop();
     delete E;
 }
 
@@ -468,7 +471,7 @@ static glac_status ens_links(glac_ensemble *E, int i, double *host, bool set) {
             E->staging_cap = bytes;
         }
         if (set) {
-            eck(cudaMemcpyAsync(E->staging, host, bytes, cudaMemcpyHostToDevice, E->stream), "H2D");
+            eck(copy_to_device(E->staging, host, bytes, E->d.device, E->stream), "H2D");
             if (E->d.precision == GLAC_FP64) launch_aos_to_soa(E->geo[i], E->staging, field_of<double>(E, 0, i), E->stream);
             else launch_aos_to_soa(E->geo[i], E->staging, field_of<float>(E, 0, i), E->stream);
             eck(cudaGetLastError(), "layout");
@@ -481,7 +484,7 @@ static glac_status ens_links(glac_ensemble *E, int i, double *host, bool set) {
             else launch_soa_to_aos(E->geo[i], field_of<float>(E, 0, i), E->staging, E->stream);
             eck(cudaGetLastError(), "layout");
             E->launches++;
-            eck(cudaMemcpyAsync(host, E->staging, bytes, cudaMemcpyDeviceToHost, E->stream), "D2H");
+            eck(copy_to_host(host, E->staging, bytes, E->d.device, E->stream), "D2H");
         }
         eck(cudaStreamSynchronize(E->stream), "sync");
         return GLAC_OK;

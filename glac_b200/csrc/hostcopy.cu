@@ -1,0 +1,151 @@
+// The driver copies pageable memory through one thread, at 11 GB/s each way on a
+// B200 host, and a fresh array's first touch falls to the same thread (382 MB
+// down into a new array: 82 ms), where the link moves 55 GB/s.  Here each of up
+// to eight threads moves every eighth 1 MB piece through two pinned buffers of
+// its own, so that pieces are copied (and touched) in parallel and beside the
+// transfers of others.  Copies below kSplitBytes, copies of memory that is
+// already pinned, and copies while another thread has the buffers go the plain way.
+// Upload / download / download into a new array on a 16-core host: 382 MB 34.6 /
+// 19.8 / 82 ms plain, 8.8 / 10.1 / 19.4 so; 24 MB 1.25 / 1.26 / 1.23 and 0.85 / 0.76 / 0.78.
+#include "hostcopy.cuh"
+
+#include <algorithm>
+#include <atomic>
+#include <cstring>
+#include <mutex>
+#include <system_error>
+#include <thread>
+
+namespace glac {
+
+namespace {
+
+constexpr size_t kPiece = (size_t)1 << 20;
+constexpr int kThreads = 8, kSlots = 2;
+// two pieces a thread: below, starting the threads costs what they save
+constexpr size_t kSplitBytes = 16 * kPiece;
+
+std::mutex g_hold_mu;   // g_holders and the buffers' lifetime
+int g_holders = 0;
+std::mutex g_use_mu;    // one transfer at a time
+char *g_pinned = nullptr;
+
+bool pageable(const void *host) {
+    cudaPointerAttributes a;
+    if (cudaPointerGetAttributes(&a, host) != cudaSuccess) {
+        cudaGetLastError();
+        return true;
+    }
+    return a.type == cudaMemoryTypeUnregistered;
+}
+
+// Piece `c` of the copy by thread k's slot; `to_device` picks the direction.
+cudaError_t worker(int k, int threads, char *dev, char *host, size_t bytes, int device, cudaStream_t st,
+                   bool to_device, std::atomic<int> *failed) {
+    cudaError_t e = cudaSetDevice(device);
+    cudaEvent_t ev[kSlots] = {nullptr, nullptr};
+    for (int i = 0; i < kSlots && e == cudaSuccess; i++) e = cudaEventCreateWithFlags(&ev[i], cudaEventDisableTiming);
+    const size_t pieces = (bytes + kPiece - 1) / kPiece;
+    auto size = [&](size_t c) { return std::min(kPiece, bytes - c * kPiece); };
+    auto slot = [&](int i) { return g_pinned + ((size_t)k * kSlots + i) * kPiece; };
+    // pending[i]: the piece whose transfer uses slot i
+    size_t pending[kSlots];
+    bool busy[kSlots] = {false, false};
+    auto finish = [&](int i) {
+        if (!busy[i]) return;
+        const cudaError_t w = cudaEventSynchronize(ev[i]);
+        if (e == cudaSuccess) e = w;
+        if (!to_device && e == cudaSuccess) memcpy(host + pending[i] * kPiece, slot(i), size(pending[i]));
+        busy[i] = false;
+    };
+    int i = 0;
+    for (size_t c = k; c < pieces && e == cudaSuccess && !failed->load(); c += threads, i ^= 1) {
+        finish(i);
+        if (e != cudaSuccess) break;
+        if (to_device) memcpy(slot(i), host + c * kPiece, size(c));
+        e = to_device ? cudaMemcpyAsync(dev + c * kPiece, slot(i), size(c), cudaMemcpyHostToDevice, st)
+                      : cudaMemcpyAsync(slot(i), dev + c * kPiece, size(c), cudaMemcpyDeviceToHost, st);
+        if (e != cudaSuccess) break;
+        pending[i] = c;
+        busy[i] = true;
+        const cudaError_t r = cudaEventRecord(ev[i], st);
+        if (r != cudaSuccess) {
+            cudaStreamSynchronize(st);  // the slot is not left while a transfer may use it
+            e = r;
+        }
+    }
+    finish(i);
+    finish(i ^ 1);
+    for (cudaEvent_t v : ev)
+        if (v) cudaEventDestroy(v);
+    if (e != cudaSuccess) failed->store(1);
+    return e;
+}
+
+cudaError_t split_copy(char *dev, char *host, size_t bytes, int device, cudaStream_t st, bool to_device) {
+    const int threads = (int)std::min<size_t>(
+        {(size_t)kThreads, std::max(1u, std::thread::hardware_concurrency() / 2), (bytes + kPiece - 1) / kPiece});
+    std::atomic<int> failed{0};
+    cudaError_t err[kThreads];
+    std::thread pool[kThreads];
+    int made = 1;
+    // threads that cannot be started leave their pieces to fewer: the count is fixed
+    // only once they all run
+    std::atomic<int> count{0};
+    auto run = [&](int k) {
+        int n;
+        while ((n = count.load()) == 0) std::this_thread::yield();
+        err[k] = k < n ? worker(k, n, dev, host, bytes, device, st, to_device, &failed) : cudaSuccess;
+    };
+    try {
+        for (; made < threads; made++) pool[made] = std::thread(run, made);
+    } catch (const std::system_error &) {
+    }
+    count.store(made);
+    run(0);
+    cudaError_t e = err[0];
+    for (int k = 1; k < made; k++) {
+        pool[k].join();
+        if (e == cudaSuccess) e = err[k];
+    }
+    return e;
+}
+
+cudaError_t copy(char *dev, char *host, size_t bytes, int device, cudaStream_t st, bool to_device) {
+    if (bytes >= kSplitBytes && pageable(host)) {
+        std::unique_lock<std::mutex> use(g_use_mu, std::try_to_lock);
+        if (use.owns_lock()) {
+            if (!g_pinned && cudaHostAlloc(&g_pinned, kThreads * kSlots * kPiece, cudaHostAllocPortable) != cudaSuccess) {
+                cudaGetLastError();
+                g_pinned = nullptr;
+            }
+            if (g_pinned) return split_copy(dev, host, bytes, device, st, to_device);
+        }
+    }
+    if (to_device) return cudaMemcpyAsync(dev, host, bytes, cudaMemcpyHostToDevice, st);
+    const cudaError_t e = cudaMemcpyAsync(host, dev, bytes, cudaMemcpyDeviceToHost, st);
+    return e == cudaSuccess ? cudaStreamSynchronize(st) : e;
+}
+
+}  // namespace
+
+cudaError_t copy_to_device(void *dev, const void *host, size_t bytes, int device, cudaStream_t st) {
+    return copy(static_cast<char *>(dev), static_cast<char *>(const_cast<void *>(host)), bytes, device, st, true);
+}
+cudaError_t copy_to_host(void *host, const void *dev, size_t bytes, int device, cudaStream_t st) {
+    return copy(static_cast<char *>(const_cast<void *>(dev)), static_cast<char *>(host), bytes, device, st, false);
+}
+
+void hostcopy_hold() {
+    std::lock_guard<std::mutex> lock(g_hold_mu);
+    g_holders++;
+}
+void hostcopy_drop() {
+    std::lock_guard<std::mutex> lock(g_hold_mu);
+    if (--g_holders > 0) return;
+    std::lock_guard<std::mutex> use(g_use_mu);
+    if (g_pinned) cudaFreeHost(g_pinned);
+    g_pinned = nullptr;
+}
+
+}  // namespace glac

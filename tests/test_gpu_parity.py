@@ -348,6 +348,33 @@ def test_hot_start_matches_oracle(g, oracle):
             assert L.unitarity_violation() < (1e-13 if prec == "fp64" else 1e-6)
 
 
+@pytest.mark.parametrize("nt", [16, 18, 24, 34])
+def test_large_fields_round_trip_from_several_threads(g, nt):
+    # below and above the size (16 MB) from which fields go through several host
+    # threads, none a whole number of the 1 MB pieces; two contexts at a time, of
+    # which one finds the pinned buffers taken and copies the plain way
+    import threading
+
+    N = (12, 12, 12, nt)
+    V = 12 * 12 * 12 * nt
+    fields = [np.random.default_rng(k).standard_normal((4, V, 18)) for k in range(2)]
+    bad = []
+
+    def work(k):
+        with lattice(g, N, "fp64") as L:
+            for _ in range(3):
+                L.set_links(fields[k])
+                if not np.array_equal(L.get_links(), fields[k]):
+                    bad.append(k)
+
+    threads = [threading.Thread(target=work, args=(k,)) for k in range(2)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert bad == []
+
+
 def test_set_get_roundtrip(g, oracle):
     N = (4, 6, 4, 8)
     links = oracle.haar_field(N, 5)
