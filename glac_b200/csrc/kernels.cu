@@ -759,16 +759,18 @@ __global__ void __launch_bounds__(128) k_esj(Geom g, LinkField<T> L, float beta,
     const int mu = plane >> 1, p = plane & 1, s = offset + i * stride;
     const Site n = site_from_ps(g, p, s);
     const M3<T> A = staple(L, g, n, p, mu);
-    float f[8];
-    staple_features(A, beta, f);
-    float4 *fo = reinterpret_cast<float4 *>(feat + row * 8);
-    fo[0] = make_float4(f[0], f[1], f[2], f[3]);
-    fo[1] = make_float4(f[4], f[5], f[6], f[7]);
     const uint32_t link_id = (uint32_t)mu * (uint32_t)g.V + (uint32_t)n.lex;
-    if (ids) ids[row] = link_id;
+    if (blockIdx.y == 0) {
+        float f[8];
+        staple_features(A, beta, f);
+        float4 *fo = reinterpret_cast<float4 *>(feat + row * 8);
+        fo[0] = make_float4(f[0], f[1], f[2], f[3]);
+        fo[1] = make_float4(f[4], f[5], f[6], f[7]);
+        if (ids) ids[row] = link_id;
+    }
     if (n_eps == 0) return;
     const M3<T> W0 = mul(L.load(mu, p, s), A);
-    for (int k = 0; k < n_eps; k++) {
+    for (int k = blockIdx.y; k < n_eps; k += gridDim.y) {
         const T eps = (T)eps_grid[k], sq = sqrt(T(1) - eps * eps);
         T J = T(0);
         for (int tr = 0; tr < trials; tr++) {
@@ -797,10 +799,19 @@ void launch_esj(const Geom &g, const LinkField<T> &L, double beta, int nhits, in
                 int trials, int stride, int offset, int ns, uint64_t seed, uint32_t snapshot, uint32_t stream_id,
                 bool flips, float *feat, float *esj, uint32_t *ids, cudaStream_t st) {
     const long long rows = 8ll * ns;
-    k_esj<T><<<(unsigned)((rows + 127) / 128), 128, 0, st>>>(g, L, (float)beta, (T)(-beta / 3.0), nhits, n_eps,
-                                                            eps_grid_dev, trials, stride, offset, ns, (uint32_t)seed,
-                                                            (uint32_t)(seed >> 32), snapshot,
-                                                            stream_id | 0x80000000u, flips, feat, esj, ids);
+    const unsigned gx = (unsigned)((rows + 127) / 128);
+    // Spreads of a row are independent, and a snapshot has fewer rows than the GPU
+    // has thread slots: they go over as many blocks as fill it about twice
+    // (148 SMs x 4 blocks), each of which forms the staple again.  16 spreads x 4
+    // trials x 10 hits on B200, one thread a row / so: 2,048 rows FP32 357 / 68 us,
+    // FP64 1712 / 100; 41,472 rows FP32 766 / 585, FP64 3658 / 1086 (which has the
+    // divisions of its proposals removed as well).
+    long long gy = n_eps < 1 ? 1 : (2 * 148 * 4 + gx - 1) / gx;
+    if (gy > n_eps && n_eps > 0) gy = n_eps;
+    k_esj<T><<<dim3(gx, (unsigned)gy), 128, 0, st>>>(g, L, (float)beta, (T)(-beta / 3.0), nhits, n_eps, eps_grid_dev,
+                                                     trials, stride, offset, ns, (uint32_t)seed,
+                                                     (uint32_t)(seed >> 32), snapshot, stream_id | 0x80000000u, flips,
+                                                     feat, esj, ids);
 }
 template void launch_esj<double>(const Geom &, const LinkField<double> &, double, int, int, const float *, int, int,
                                  int, int, uint64_t, uint32_t, uint32_t, bool, float *, float *, uint32_t *,

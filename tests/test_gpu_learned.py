@@ -99,6 +99,22 @@ def test_esj_matches_oracle(g, torch, oracle, prec, flips):
         assert abs(esj.mean() - want.mean()) < 0.01 * want.mean()
 
 
+@pytest.mark.parametrize("prec", ["fp64", "fp32"])
+@pytest.mark.parametrize("stride", [8, 64, 4096])
+def test_esj_rows_do_not_depend_on_the_sample(g, torch, prec, stride):
+    # a link's row is the same bits whether one thread takes all its spreads
+    # (every link sampled) or they go over 3, 16 or 16 of 16 blocks of a thinner sample
+    grid = np.geomspace(0.05, 0.8, 16)
+    with g.Lattice((16, 16, 16, 32), beta=6.0, precision=prec, seed=3, n_updates=2) as L:
+        L.hot_start(2)
+        L.metropolis(2)
+        fa, ja, ia = esj_rows(g, torch, L, grid, 1, 1, 0)
+        fb, jb, ib = esj_rows(g, torch, L, grid, 1, stride, 0)
+    at = np.argsort(ia)[np.searchsorted(np.sort(ia), ib)]
+    assert np.array_equal(ia[at], ib)
+    assert np.array_equal(ja[at], jb) and np.array_equal(fa[at], fb)
+
+
 @pytest.mark.parametrize("mode,n", [(0, 3000), (1, 3000), (1, 200_000)])
 def test_forward_matches_oracle(g, torch, learned, mode, n):
     # mode 0: the sampler's warp routine; mode 1: tcgen05 tensor-core tiles of
