@@ -179,6 +179,8 @@ template <> struct LinkField<double> {
 #pragma unroll
         for (int k = 0; k < 9; k++) b[32 * k] = make_double2(U.e[k].re, U.e[k].im);
     }
+    // element e of a link
+    __device__ __forceinline__ double2 *element(int mu, int par, int s, int e) const { return p + base(mu, par, s) + 32 * e; }
 };
 
 template <> struct LinkField<float> {
@@ -219,6 +221,10 @@ template <> struct LinkField<float> {
         for (int k = 0; k < 4; k++)
             b[32 * k] = make_float4(U.e[2 * k].re, U.e[2 * k].im, U.e[2 * k + 1].re, U.e[2 * k + 1].im);
         p2[at2(mu, par, s)] = make_float2(U.e[8].re, U.e[8].im);
+    }
+    __device__ __forceinline__ float2 *element(int mu, int par, int s, int e) const {
+        if (e == 8) return p2 + at2(mu, par, s);
+        return reinterpret_cast<float2 *>(p4 + base4(mu, par, s) + 32 * (e >> 1)) + (e & 1);
     }
 };
 

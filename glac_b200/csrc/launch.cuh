@@ -20,11 +20,14 @@ namespace glac {
 __device__ __forceinline__ void chain_wait() { cudaGridDependencySynchronize(); }
 __device__ __forceinline__ void chain_release() { cudaTriggerProgrammaticLaunchCompletion(); }
 
+// `shared`: dynamic shared memory of a block in bytes
 template <typename... Params, typename... Args>
-void launch_chained(void (*kernel)(Params...), unsigned grid, unsigned threads, cudaStream_t st, Args... args) {
+void launch_chained_shared(void (*kernel)(Params...), unsigned grid, unsigned threads, size_t shared, cudaStream_t st,
+                           Args... args) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(grid);
     cfg.blockDim = dim3(threads);
+    cfg.dynamicSmemBytes = shared;
     cfg.stream = st;
     cudaLaunchAttribute at = {};
     at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
@@ -32,6 +35,10 @@ void launch_chained(void (*kernel)(Params...), unsigned grid, unsigned threads, 
     cfg.attrs = &at;
     cfg.numAttrs = 1;
     cudaLaunchKernelEx(&cfg, kernel, static_cast<Params>(args)...);
+}
+template <typename... Params, typename... Args>
+void launch_chained(void (*kernel)(Params...), unsigned grid, unsigned threads, cudaStream_t st, Args... args) {
+    launch_chained_shared(kernel, grid, threads, 0, st, args...);
 }
 
 }  // namespace glac

@@ -321,6 +321,32 @@ def test_accept_decisions_full_reference_sweep(g, oracle, reference):
     assert rel_err(final, tr["links"]) < 1e-13
 
 
+@pytest.mark.parametrize("prec", ["fp64", "fp32"])
+@pytest.mark.parametrize("learned", [False, True])
+@pytest.mark.parametrize("N, hits", [((4, 4, 4, 4), 10), ((10, 6, 4, 6), 23), ((4, 6, 6, 6), 0), ((6, 4, 6, 8), 1),
+                                     ((8, 8, 8, 36), 10), ((8, 8, 8, 38), 10)])
+def test_small_lattice_sweeps_are_bit_identical(g, prec, learned, N, hits):
+    # the kernel that gives each link of a small lattice eight warps (up to 18,944
+    # sites) does the operations of the one-thread kernel (variant 1) in their
+    # order: planes with a ragged last block, no hits, and hits in batches of ten
+    # with a remainder give the same chain bit for bit
+    rng = np.random.default_rng(1)
+    P = np.zeros(g.MLP_NPARAMS, np.float32)
+    P[0:256] = rng.standard_normal(256) * 0.5
+    P[288:1312] = rng.standard_normal(1024) * 0.25
+    P[1344:1376] = rng.standard_normal(32) * 0.3
+    out = []
+    for variant in (0, 1):
+        with lattice(g, N, prec, beta=6.0, n_updates=hits, seed=8) as L:
+            L.tuning = [0, variant, 0]
+            if learned:
+                L.set_proposal_net(P, 0.1, 0.6)
+            L.hot_start(3)
+            out.append((L.metropolis(2), L.get_links()))
+    assert out[0][0] == out[1][0]
+    assert np.array_equal(out[0][1], out[1][1])
+
+
 @pytest.mark.parametrize("flips", [True, False])
 def test_checkerboard_sweep_matches_oracle(g, oracle, flips):
     N = (4, 4, 4, 8)
