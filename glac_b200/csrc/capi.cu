@@ -215,13 +215,20 @@ void measure_into(glac_ctx *c, double *dev_out) {
     c->launches += 3;
 }
 
-void ensure_flow_partial(glac_ctx *c, size_t n) {
-    if (c->flow_partial_cap >= n) return;
-    if (c->flow_partial) cudaFree(c->flow_partial);
-    c->flow_partial = nullptr;
-    c->flow_partial_cap = 0;
-    ck(cudaMalloc(&c->flow_partial, n * sizeof(double)), "cudaMalloc flow partials");
-    c->flow_partial_cap = n;
+// Room for the partial sums of as many measurements as 16 MB hold (at least one,
+// at most 256), made once, whatever the length of the flow; returns how many.
+int ensure_flow_partial(glac_ctx *c, size_t row) {
+    size_t rows = ((size_t)16 << 20) / (row * sizeof(double));
+    rows = rows < 1 ? 1 : rows > 256 ? 256 : rows;
+    const size_t n = rows * row;
+    if (c->flow_partial_cap < n) {
+        if (c->flow_partial) cudaFree(c->flow_partial);
+        c->flow_partial = nullptr;
+        c->flow_partial_cap = 0;
+        ck(cudaMalloc(&c->flow_partial, n * sizeof(double)), "cudaMalloc flow partials");
+        c->flow_partial_cap = n;
+    }
+    return (int)rows;
 }
 
 // One Luscher RK3 step: three fused stages, cur -> other -> cur -> other.
@@ -654,15 +661,11 @@ glac_status glac_flow(glac_ctx *c, int n_steps, double *obs) {
         // own; the last one always a pass of its own.
         const bool fused = obs && fused_measure_usable(c);
         const FlowMode mode = flow_mode(c);
-        int rows = 1;  // measurements whose partial sums wait for one final reduction (16 MB at most)
+        int rows = 1;  // measurements whose partial sums wait for one final reduction
         if (obs) {
             ensure_obs(c, per * (size_t)(n_steps + 1));
             if (!fused || n_steps == 0) measure_into(c, c->obs_dev);
-            if (fused && n_steps > 0) {
-                const size_t fit = ((size_t)16 << 20) / (mode.row * sizeof(double));
-                rows = fit < 1 ? 1 : fit > (size_t)n_steps ? n_steps : (int)fit;
-                ensure_flow_partial(c, rows * mode.row);
-            }
+            if (fused && n_steps > 0) rows = ensure_flow_partial(c, mode.row);
         }
         for (int i = 0; i < n_steps; i++) {
             const int r = i % rows;
