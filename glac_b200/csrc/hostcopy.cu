@@ -22,8 +22,9 @@ namespace {
 
 constexpr size_t kPiece = (size_t)1 << 20;
 constexpr int kThreads = 8, kSlots = 2;
-// two pieces a thread: below, starting the threads costs what they save
-constexpr size_t kSplitBytes = 16 * kPiece;
+// a piece for each thread: below, starting the threads costs what they save
+// (4.7 MB 270 us plain, 285 so; 9.2 MB 500 / 470; 15.9 MB 840 / 650)
+constexpr size_t kSplitBytes = kThreads * kPiece;
 
 std::mutex g_hold_mu;   // g_holders and the buffers' lifetime
 int g_holders = 0;

@@ -374,9 +374,9 @@ def test_hot_start_matches_oracle(g, oracle):
             assert L.unitarity_violation() < (1e-13 if prec == "fp64" else 1e-6)
 
 
-@pytest.mark.parametrize("nt", [16, 18, 24, 34])
+@pytest.mark.parametrize("nt", [8, 10, 18, 34])
 def test_large_fields_round_trip_from_several_threads(g, nt):
-    # below and above the size (16 MB) from which fields go through several host
+    # below and above the size (8 MB) from which fields go through several host
     # threads, none a whole number of the 1 MB pieces; two contexts at a time, of
     # which one finds the pinned buffers taken and copies the plain way
     import threading
