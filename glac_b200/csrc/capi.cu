@@ -169,8 +169,8 @@ struct FlowMode {
 // option or tuning: up to one and a half times the thread slots of a link per
 // thread (148 SMs x 24 warps in FP32), in FP64 once (x 16 warps), beyond which
 // its idle warps cost more than its shorter chain gives.  Microseconds per
-// measured step on B200, split / a thread per link: FP32 8^3 x 16 16.9 / 22.0,
-// 12^3 x 24 57 / 60, 14^3 x 28 108 / 101; FP64 8^3 x 16 33 / 36, 10^3 x 20
+// measured step on B200, split / a thread per link: FP32 8^3 x 16 18 / 22,
+// 12^3 x 24 57 / 60, 14^3 x 28 108 / 101; FP64 8^3 x 16 31 / 36, 10^3 x 20
 // 74 / 74, 12^3 x 24 125 / 120.
 constexpr int kSplitMaxSitesFp32 = 148 * 24 * 32 * 3 / 2 / 4, kSplitMaxSitesFp64 = 148 * 16 * 32 / 4;
 FlowMode flow_mode(const glac_ctx *c) {

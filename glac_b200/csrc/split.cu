@@ -51,8 +51,10 @@ template <> struct LaneSlots<double> {
 // MEAS (stage 0): the clover parts of the input field, as k_flow_stage0_meas.
 // COMBINE (stage 1): the blocks of direction 0 also combine the parts of their
 // 32 sites into the partial sums of a 32-site plan.
+// Eight (FP32) and five (FP64) blocks of three warps per SM; FP64's measured stage 0,
+// which spills 180 B so, four: 31.0 us per measured step of 8^3 x 16 on B200, not 32.9.
 template <typename T, int STAGE, bool MEAS, bool COMBINE>
-__global__ void __launch_bounds__(32 * kSplitWarps, sizeof(T) == 4 ? 8 : 5)
+__global__ void __launch_bounds__(32 * kSplitWarps, sizeof(T) == 4 ? 8 : MEAS ? 4 : 5)
     k_flow_split(Geom g, LinkField<T> in, LinkField<T> out, ForceField<T> zf, T alpha, T beta, CloverParts<T> cp,
                  double *partial) {
     __shared__ LaneSlots<T> slot;
