@@ -586,9 +586,12 @@ static void metro_dispatch(int regs, dim3 grid, cudaStream_t st, const Geom &g, 
 // 128 (four) where a fifth block finds no work, up to one wave of blocks, and for
 // the learned spread, whose kernel spills at 96.  Microseconds per sweep on B200
 // at 128 / 96: 12^3 x 24 112 / 115, 24^3 x 48 788 / 778, 32^3 x 64 2276 / 2248;
-// learned 24^3 x 48 898 / 934 (uncapped 930).
+// learned 24^3 x 48 898 / 934 (uncapped 930).  FP64's default is uncapped (three
+// blocks per SM), but 128 with a small spill from ten blocks per SM on: 16^3 x 32
+// 347 / 331 us, 24^3 x 48 1463 / 1498, 32^3 x 64 4310 / 4432.
 static int metro_regs(bool fp32, int variant, bool learned, int blocks) {
     if (fp32 && variant == 0 && (learned || blocks <= 5 * 148)) return 128;
+    if (!fp32 && variant == 0 && blocks > 10 * 148) return 128;
     return variant_regs(FAM_METRO, fp32, variant);
 }
 

@@ -38,26 +38,17 @@ __device__ __forceinline__ M3<T> staple(const LinkField<T> &L, const Geom &g, co
     M3<T> A;
     set_zero(A);
     const int q = p ^ 1;
-    // Neighbour indices: select chains (pick4) in FP32 and in the flow stage,
-    // indexed arrays in the FP64 Metropolis kernel; each form is the faster one
-    // there (FP64 flow stage at 128 registers, 24^3 x 48 on B200: 423 against 449 us).
-    constexpr bool sel = sizeof(T) == 4 || RECON;
-    const int f_mu = sel ? step_offset(g, n, mu, +1) : step_offset_indexed(g, n, mu, +1);
+    // Neighbour indices by select chains (pick4): indexed arrays put the site and
+    // the lattice in local memory (FP64 on B200, indexed / so: flow stage 24^3 x 48
+    // 449 / 423 us, Metropolis sweep 24^3 x 48 1549 / 1498, 16^3 x 32 343 / 331).
+    const int f_mu = step_offset(g, n, mu, +1);
     const int s_mu = (n.lex + f_mu) >> 1;
 #pragma unroll(UNROLL ? 4 : 1)
     for (int nu = 0; nu < 4; nu++) {
         if (nu == mu) continue;
-        int s_nup, s_num, s_diag;
-        if constexpr (sel) {
-            const int b_nu = step_offset(g, n, nu, -1);
-            s_nup = (n.lex + step_offset(g, n, nu, +1)) >> 1;
-            s_num = (n.lex + b_nu) >> 1;
-            s_diag = (n.lex + f_mu + b_nu) >> 1;
-        } else {
-            s_nup = lex_step(g, n, nu, +1) >> 1;
-            s_num = lex_step(g, n, nu, -1) >> 1;
-            s_diag = lex_step2(g, n, mu, +1, nu, -1) >> 1;
-        }
+        const int b_nu = step_offset(g, n, nu, -1);
+        const int s_nup = (n.lex + step_offset(g, n, nu, +1)) >> 1, s_num = (n.lex + b_nu) >> 1,
+                  s_diag = (n.lex + f_mu + b_nu) >> 1;
         {
             M3<T> a = L.load(nu, q, s_mu);
             M3<T> b = L.load(mu, q, s_nup);

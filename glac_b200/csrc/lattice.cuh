@@ -106,8 +106,8 @@ GLAC_HD int lex_step2(const Geom &g, const Site &n, int d, int a, int e, int b) 
 // v[d] for a direction d that may be a run-time value, as a chain of selects:
 // the arrays stay in registers, where indexing them with a run-time d places
 // the Site and the Geom in local memory.  Folds to v[d] for a constant d.  The
-// FP32 staple and both flow stages run faster with it; the FP64 Metropolis
-// staple and the clover run faster with the indexed form above (timed on B200).
+// staples run faster with it, the ensemble's clover with the indexed form above
+// (timed on B200).
 GLAC_HD int pick4(const int v[4], int d) { return d == 0 ? v[0] : d == 1 ? v[1] : d == 2 ? v[2] : v[3]; }
 
 // periodic offset of one step a = +1 or -1 along d, selected without indexing
