@@ -61,16 +61,8 @@ void ck(cudaError_t e, const char *what) {
 }
 void ck_launch(const char *what) { ck(cudaGetLastError(), what); }
 
-// 8 planes of Vh32 tiled sites (see lattice.cuh); FP32 adds the plain float2 plane array.
-size_t field_bytes(const glac_desc &d, const Geom &g) {
-    const size_t vh32 = (size_t)round32(g.Vh);
-    if (d.precision == GLAC_FP64) return 8 * vh32 * 9 * sizeof(double2);
-    return 8 * vh32 * 4 * sizeof(float4) + 8 * vh32 * sizeof(float2);
-}
-size_t force_bytes(const glac_desc &d, const Geom &g) {
-    const size_t vh32 = (size_t)round32(g.Vh);
-    return d.precision == GLAC_FP64 ? 8 * vh32 * 4 * sizeof(double2) : 8 * vh32 * 2 * sizeof(float4);
-}
+size_t field_bytes(const glac_desc &d, const Geom &g) { return glac::field_bytes(g.Vh, d.precision == GLAC_FP64); }
+size_t force_bytes(const glac_desc &d, const Geom &g) { return glac::force_bytes(g.Vh, d.precision == GLAC_FP64); }
 
 LinkField<double> f64(glac_ctx *c, int i) {
     LinkField<double> L;
@@ -191,17 +183,10 @@ template <typename T> ForceField<T> force_field(glac_ctx *c) {
     if constexpr (sizeof(T) == 8) return z64(c);
     else return z32(c);
 }
-// The stand-alone measurement's parts: slots 0-8 in the field that is not
-// current, the others and the plaquettes in the force (neither holds anything
-// between flow steps).
+// The stand-alone measurement's parts, in the field that is not current and in
+// the force (neither holds anything between flow steps).
 template <typename T> PlaneParts<T> plane_parts(glac_ctx *c) {
-    PlaneParts<T> v;
-    v.lo.p = reinterpret_cast<decltype(v.lo.p)>(c->field[c->cur ^ 1]);
-    v.hi.p = reinterpret_cast<decltype(v.hi.p)>(c->force);
-    v.lo.Vh = v.hi.Vh = c->g.Vh;
-    v.lo.Vh32 = v.hi.Vh32 = round32(c->g.Vh);
-    v.plaq = reinterpret_cast<T *>(static_cast<char *>(c->force) + force_bytes(c->d, c->g) / 4 * 3);
-    return v;
+    return plane_parts_view<T>(c->field[c->cur ^ 1], c->force, c->g.Vh);
 }
 
 void measure_into(glac_ctx *c, double *dev_out) {

@@ -284,21 +284,44 @@ template <typename T> struct CloverParts {
     T *plaq;
 };
 
+// Bytes of a link field (8 planes of Vh32 tiled sites, FP32 with the plain float2
+// planes behind them) and of a force.
+inline size_t field_bytes(int Vh, bool fp64) {
+    const size_t vh32 = (size_t)round32(Vh);
+    return fp64 ? 8 * vh32 * 9 * sizeof(double2) : 8 * vh32 * 4 * sizeof(float4) + 8 * (size_t)Vh * sizeof(float2);
+}
+inline size_t force_bytes(int Vh, bool fp64) {
+    const size_t vh32 = (size_t)round32(Vh);
+    return fp64 ? 8 * vh32 * 4 * sizeof(double2) : 8 * vh32 * 2 * sizeof(float4);
+}
+
 // The same twelve slots for the stand-alone measurement, in two buffers: slots
-// 0-8 in one the size of a link field, 9-11 and six plaquettes per site,
-// plaq[(plane * 2 + parity) * Vh + s], in one the size of a force (9 x 8 reals are
-// 4 x 18, and 3 x 8 + 6 fewer than 4 x 8).
+// 0-7 and, behind them, six plaquettes per site, plaq[(plane * 2 + parity) * Vh + s],
+// in one the size of a link field (8 x 8 + 6 reals of 4 x 18), slots 8-11 in one
+// the size of a force.  Eight slots reach as far as the four tiled directions of
+// an FP32 field (four FP64 directions reach further), so their 32-bit offsets
+// hold wherever a field's do (field_offsets_fit).
 template <typename T> struct PlaneParts {
+    static constexpr int kLow = 8;
     ForceField<T> lo, hi;
     T *plaq;
     __device__ __forceinline__ AH8<T> load(int k, int par, int s) const {
-        return k < 9 ? lo.load(k, par, s) : hi.load(k - 9, par, s);
+        return k < kLow ? lo.load(k, par, s) : hi.load(k - kLow, par, s);
     }
     __device__ __forceinline__ void store(int k, int par, int s, const AH8<T> &Z) const {
-        if (k < 9) lo.store(k, par, s, Z);
-        else hi.store(k - 9, par, s, Z);
+        if (k < kLow) lo.store(k, par, s, Z);
+        else hi.store(k - kLow, par, s, Z);
     }
 };
+template <typename T> PlaneParts<T> plane_parts_view(void *field, void *force, int Vh) {
+    PlaneParts<T> v;
+    v.lo.p = reinterpret_cast<decltype(v.lo.p)>(field);
+    v.hi.p = reinterpret_cast<decltype(v.hi.p)>(force);
+    v.lo.Vh = v.hi.Vh = Vh;
+    v.lo.Vh32 = v.hi.Vh32 = round32(Vh);
+    v.plaq = reinterpret_cast<T *>(field) + (size_t)PlaneParts<T>::kLow * 2 * 8 * round32(Vh);
+    return v;
+}
 
 // ---------------------------------------------------------------------------
 // Philox4x32-10 (Salmon, Moraes, Dror, Shaw, SC'11)

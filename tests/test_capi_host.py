@@ -117,3 +117,27 @@ def test_ensemble_draw_is_seeded_and_uneven():
     assert d1 == d2 and b1 == b2 and len(d1) == 64
     assert set(d1) <= set(SIZES) and set(b1) <= set(BETAS)
     assert len(set(d1)) == 4 and len(set(b1)) == 4  # every size and coupling occurs
+
+
+@pytest.fixture(scope="module")
+def parts_layout(tmp_path_factory):
+    import subprocess
+    exe = str(tmp_path_factory.mktemp("native") / "parts_layout")
+    cuda = os.environ.get("CUDA_HOME", "/usr/local/cuda")
+    subprocess.run(["g++", "-std=c++17", "-O1", "-I", os.path.join(cuda, "include"), "-I",
+                    os.path.join(ROOT, "glac_b200", "csrc"), os.path.join(ROOT, "tests", "native", "parts_layout.cpp"),
+                    "-o", exe], check=True)
+    return lambda V: [line.split() for line in subprocess.run([exe, str(V)], check=True, capture_output=True,
+                                                              text=True).stdout.splitlines()]
+
+
+@pytest.mark.parametrize("V, fp32, fp64", [
+    (4 * 4 * 4 * 4, True, True), (4 * 6 * 6 * 6, True, True), (10 * 6 * 4 * 6, True, True),
+    (128 * 128 * 128 * 56, True, True),    # the largest of 128^3 in FP64
+    (128 * 128 * 128 * 112, True, False),  # below and above 2^32 / 36 x 2 sites, where a ninth
+    (128 * 128 * 128 * 114, True, False),  # slot of a field would leave the 32-bit offsets
+    (128 * 128 * 128 * 126, True, False),  # the largest of 128^3 in FP32
+    (128 * 128 * 128 * 128, False, False)])
+def test_measurement_parts_fit_the_fields_they_lie_in(parts_layout, V, fp32, fp64):
+    # every slot's offsets, for every lattice that a context takes
+    assert parts_layout(V) == [["fp32", "1", str(int(fp32))], ["fp64", "1", str(int(fp64))]]
