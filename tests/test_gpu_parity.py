@@ -504,6 +504,35 @@ def test_weinberg_matches_reference(g, oracle, reference, prec, tol):
         assert_obs_close(np.r_[got[:3], got[4:12]], base, 1e-12, "weinberg vs plain sampler")
 
 
+@pytest.mark.parametrize("prec", ["fp64", "fp32"])
+@pytest.mark.parametrize("N", [(4, 4, 4, 4), (4, 6, 6, 6), (6, 4, 6, 8), (10, 6, 4, 6), (8, 8, 4, 16), (16, 16, 16, 4)])
+def test_weinberg_and_densities_match_oracle(g, oracle, prec, N):
+    # half slices of less than a warp's sites, of one block (whole and ragged
+    # warps) and of many.  Plaquette and energy against their own values.  Charges
+    # cancel over sites, so a density is held against the largest density, a
+    # slice's sum against the largest slice, and a total against the sum of the
+    # slices' magnitudes, each by the precision's bar.
+    links = oracle.flow(N, oracle.haar_field(N, 29), 0.02, 3)
+    want, (wq, we) = oracle.weinberg(N, links), oracle.density(N, links)
+    tol, nt = TOL[prec], N[3]
+    with lattice(g, N, prec) as L:
+        L.set_links(links)
+        got = L.measure_weinberg()
+        obs, q, e = L.measure_density()
+        base = L.measure()
+        assert np.array_equal(L.measure_weinberg(), got)  # scratch of the one does not reach the other
+    for k in (0, 2):
+        assert abs(got[k] - want[k]) <= tol * abs(want[k])
+    for total, sl in ((1, slice(4, 4 + nt)), (3, slice(4 + nt, 4 + 2 * nt))):
+        assert np.max(np.abs(got[sl] - want[sl])) <= tol * np.max(np.abs(want[sl]))
+        assert abs(got[total] - want[total]) <= tol * np.sum(np.abs(want[sl]))
+    assert np.max(np.abs(q - wq)) <= tol * np.max(np.abs(wq))
+    assert np.max(np.abs(e - we)) <= tol * np.max(np.abs(we))
+    # the same FP64 sums in all three entry points
+    for other in (obs, base):
+        assert np.max(np.abs(other - np.r_[got[:3], got[4:4 + nt]])) <= 1e-12 * np.sum(np.abs(other))
+
+
 def test_observables_at_the_largest_time_extent(g, oracle):
     # Nt = 1024 fills the per-slice arrays of the reduction; larger Nt is rejected at creation
     N = (4, 4, 4, 1024)
