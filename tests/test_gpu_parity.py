@@ -533,6 +533,25 @@ def test_weinberg_and_densities_match_oracle(g, oracle, prec, N):
         assert np.max(np.abs(other - np.r_[got[:3], got[4:4 + nt]])) <= 1e-12 * np.sum(np.abs(other))
 
 
+@pytest.mark.parametrize("prec", ["fp64", "fp32"])
+@pytest.mark.parametrize("N, variant, steps", [((4, 4, 4, 4), 0, 517), ((4, 4, 4, 4), 1, 517), ((4, 6, 6, 6), 0, 300),
+                                               ((24, 24, 24, 48), 0, 275)])
+def test_long_measured_flows(g, prec, N, variant, steps):
+    # partial sums are reduced 256 measurements (24^3 x 48: 134) at a time: rows
+    # past the first batch are the bits that short flows of the same field give
+    with lattice(g, N, prec, seed=6) as A, lattice(g, N, prec, seed=6) as B:
+        for L in (A, B):
+            L.tuning = [variant, 0, 0]
+            L.hot_start(4)
+        rows, left = [], steps
+        while left:
+            k = min(left, 50)
+            rows.append(B.flow(k)[:k if left > k else k + 1])
+            left -= k
+        assert np.array_equal(A.flow(steps), np.concatenate(rows))
+        assert np.array_equal(A.get_links(), B.get_links())
+
+
 def test_observables_at_the_largest_time_extent(g, oracle):
     # Nt = 1024 fills the per-slice arrays of the reduction; larger Nt is rejected at creation
     N = (4, 4, 4, 1024)
