@@ -13,7 +13,6 @@
 #include <atomic>
 #include <cstring>
 #include <mutex>
-#include <system_error>
 #include <thread>
 
 namespace glac {
@@ -90,8 +89,8 @@ cudaError_t split_copy(char *dev, char *host, size_t bytes, int device, cudaStre
     cudaError_t err[kThreads];
     std::thread pool[kThreads];
     int made = 1;
-    // threads that cannot be started leave their pieces to fewer: the count is fixed
-    // only once they all run
+    // threads that cannot be started, for want of a thread or of memory, leave their
+    // pieces to fewer: the count is fixed only once they all run
     std::atomic<int> count{0};
     auto run = [&](int k) {
         int n;
@@ -100,7 +99,7 @@ cudaError_t split_copy(char *dev, char *host, size_t bytes, int device, cudaStre
     };
     try {
         for (; made < threads; made++) pool[made] = std::thread(run, made);
-    } catch (const std::system_error &) {
+    } catch (...) {
     }
     count.store(made);
     run(0);
