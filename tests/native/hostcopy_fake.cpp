@@ -1,30 +1,34 @@
 // The host side of the field copies (hostcopy.cu) on a fake CUDA runtime whose
 // copies are memcpy.  argv: hardware threads, then one step after another:
 //   up N | down N    a copy of N bytes, checked; prints the number of transfers it took
-//   fail             from here on a thread's state finds no memory
+//   fail             the third and every later thread of the copies that follow finds no memory
 //   hold | drop      a holder comes or goes; drop prints the bytes pinned after it
 //   pinned           prints the bytes pinned now and how often memory was pinned
 #include "hostcopy.cu"
 
 #include <cstdio>
 #include <cstdlib>
-#include <map>
 #include <new>
 #include <string>
 #include <vector>
 
 static std::atomic<int> g_copies{0};
 static std::mutex g_mu;
-static std::map<void *, size_t> g_regions;
+struct Region {
+    void *p;
+    size_t n;
+};
+static Region g_regions[16];  // no allocation of the fake's own
 static int g_pins = 0;
 static unsigned g_hw = 1;
-static std::atomic<bool> g_fail{false};
-static std::thread::id g_main;
+static bool g_fail = false;         // of the main thread, which makes the threads
+static thread_local int g_left = -1;  // allocations until the first that fails; below 0: none does
 
 unsigned int std::thread::hardware_concurrency() noexcept { return g_hw; }
 
 void *operator new(size_t n) {
-    if (g_fail.load() && std::this_thread::get_id() == g_main) throw std::bad_alloc();
+    if (g_left == 0) throw std::bad_alloc();
+    if (g_left > 0) g_left--;
     if (void *p = malloc(n ? n : 1)) return p;
     throw std::bad_alloc();
 }
@@ -34,19 +38,23 @@ void operator delete(void *p, size_t) noexcept { free(p); }
 static size_t pinned() {
     std::lock_guard<std::mutex> l(g_mu);
     size_t n = 0;
-    for (auto &r : g_regions) n += r.second;
+    for (const Region &r : g_regions) n += r.n;
     return n;
 }
+static cudaError_t move(void *from, void *to, size_t n) {
+    std::lock_guard<std::mutex> l(g_mu);
+    for (Region &r : g_regions)
+        if (r.p == from) {
+            r = Region{to, n};
+            return cudaSuccess;
+        }
+    return cudaErrorInvalidValue;
+}
 static cudaError_t pin(void *p, size_t n) {
-    std::lock_guard<std::mutex> l(g_mu);
-    g_regions[p] = n;
     g_pins++;
-    return cudaSuccess;
+    return move(nullptr, p, n);
 }
-static cudaError_t unpin(void *p) {
-    std::lock_guard<std::mutex> l(g_mu);
-    return g_regions.erase(p) ? cudaSuccess : cudaErrorInvalidValue;
-}
+static cudaError_t unpin(void *p) { return move(p, nullptr, 0); }
 
 extern "C" {
 cudaError_t cudaPointerGetAttributes(cudaPointerAttributes *a, const void *) {
@@ -83,7 +91,6 @@ cudaError_t cudaThreadExchangeStreamCaptureMode(cudaStreamCaptureMode *) { retur
 }
 
 int main(int argc, char **argv) {
-    g_main = std::this_thread::get_id();
     g_hw = (unsigned)atoi(argv[1]);
     std::vector<char> dev, host;
     for (int i = 2; i < argc; i++) {
@@ -96,21 +103,20 @@ int main(int argc, char **argv) {
         } else if (s == "pinned") printf("%zu %d\n", pinned(), g_pins);
         else {
             const size_t n = (size_t)atoll(argv[++i]);
-            const bool up = s == "up", fail = g_fail.exchange(false);
+            const bool up = s == "up";
             dev.assign(n, 0);
             host.assign(n, 0);
             std::vector<char> &src = up ? host : dev;
             for (size_t k = 0; k < n; k++) src[k] = (char)(k * 31 + (k >> 11));
             g_copies = 0;
-            g_fail = fail;
+            g_left = g_fail ? 2 : -1;
             const cudaError_t e = up ? glac::copy_to_device(dev.data(), host.data(), n, 0, nullptr)
                                      : glac::copy_to_host(host.data(), dev.data(), n, 0, nullptr);
-            g_fail = false;
+            g_left = -1;
             if (e != cudaSuccess || dev != host) {
                 printf("wrong\n");
                 return 1;
             }
-            g_fail = fail;
             printf("%d\n", g_copies.load());
         }
     }
