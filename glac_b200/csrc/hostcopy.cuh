@@ -12,7 +12,7 @@ namespace glac {
 cudaError_t copy_to_device(void *dev, const void *host, size_t bytes, int device, cudaStream_t st);
 cudaError_t copy_to_host(void *host, const void *dev, size_t bytes, int device, cudaStream_t st);
 
-// The pinned staging memory (16 MB a process) lives while at least one holder does.
+// The pinned staging memory (16 MB a process, once copies pay for it) lives while at least one holder does.
 void hostcopy_hold();
 void hostcopy_drop();
 

@@ -87,7 +87,6 @@ cudaError_t cudaFreeHost(void *p) {
 }
 cudaError_t cudaHostRegister(void *p, size_t n, unsigned) { return pin(p, n); }
 cudaError_t cudaHostUnregister(void *p) { return unpin(p); }
-cudaError_t cudaThreadExchangeStreamCaptureMode(cudaStreamCaptureMode *) { return cudaSuccess; }
 }
 
 int main(int argc, char **argv) {

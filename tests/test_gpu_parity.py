@@ -401,6 +401,32 @@ def test_large_fields_round_trip_from_several_threads(g, nt):
     assert bad == []
 
 
+def test_copies_that_make_the_pinned_buffers(g):
+    # 70.8 MB fields, in two contexts at a time and again after both were closed;
+    # the one that finds the buffers taken copies the plain way
+    import threading
+
+    N = (16, 16, 16, 30)
+    V = 16 * 16 * 16 * 30
+    fields = [np.random.default_rng(k).standard_normal((4, V, 18)) for k in range(2)]
+    bad = []
+
+    def work(k):
+        with lattice(g, N, "fp64") as L:
+            for _ in range(2):
+                L.set_links(fields[k])
+                if not np.array_equal(L.get_links(), fields[k]):
+                    bad.append(k)
+
+    for _ in range(2):
+        threads = [threading.Thread(target=work, args=(k,)) for k in range(2)]
+        for t in threads:
+            t.start()
+        for t in threads:
+            t.join()
+    assert bad == []
+
+
 def test_set_get_roundtrip(g, oracle):
     N = (4, 6, 4, 8)
     links = oracle.haar_field(N, 5)

@@ -32,3 +32,27 @@ def test_no_memory_for_a_thread(fake, way):
     # a thread that cannot be made leaves its pieces to the others; 400 MB are taken
     # in pieces whatever the memory held so far
     assert fake("hold", "fail", way, 400 * MB + 7, "drop")[0][0] == 401
+
+
+PINNED = 16 * MB
+
+
+def test_short_lived_contexts_pin_nothing(fake):
+    # a context per configuration of 24 MB: pinning for its two copies would cost more than they take
+    life = ["hold", "up", 24 * MB, "down", 24 * MB, "pinned", "drop"]
+    assert fake(*(life * 4)) == [[1], [1], [0, 0], [0]] * 4
+
+
+def test_buffers_come_with_a_large_copy_and_go_with_the_last_holder(fake):
+    out = fake("hold", "hold", "up", 63 * MB, "pinned", "up", 64 * MB, "pinned", "down", 24 * MB + 1, "drop", "down",
+               80 * MB, "drop", "pinned")
+    assert out == [[1], [0, 0], [64], [PINNED, 1], [25], [PINNED], [80], [0], [0, 1]]
+
+
+def test_buffers_come_after_enough_small_copies(fake):
+    # 40 MB at a time: the seventh copy passes 256 MB; what small copies moved counts from the last holder's end
+    seven = ["up", 40 * MB] * 3 + ["down", 40 * MB] * 3 + ["pinned", "up", 40 * MB, "pinned"]
+    before, after = [[1]] * 6 + [[0, 0]], [[40], [PINNED, 1]]
+    assert fake("hold", *seven, "drop") == before + after + [[0]]
+    part = ["hold", *seven[:12], "drop"]
+    assert fake(*part, *part) == ([[1]] * 6 + [[0]]) * 2
