@@ -3,7 +3,7 @@
 // down into a new array: 82 ms), where the link moves 55 GB/s.  Here each of up
 // to eight threads moves every eighth 1 MB piece through two pinned buffers of
 // its own, so that pieces are copied (and touched) in parallel and beside the
-// transfers of others.  Copies below kSplitBytes, copies of memory that is
+// transfers of others.  Small copies (split_bytes), copies of memory that is
 // already pinned, and copies while another thread has the buffers go the plain way.
 // Upload / download / download into a new array on a 16-core host: 382 MB 34.6 /
 // 19.8 / 82 ms plain, 8.8 / 10.1 / 19.4 so; 24 MB 1.25 / 1.26 / 1.23 and 0.85 / 0.76 / 0.78.
@@ -16,6 +16,7 @@
 #include <mutex>
 #include <thread>
 
+#include <sched.h>
 #include <sys/mman.h>
 
 namespace glac {
@@ -24,9 +25,7 @@ namespace {
 
 constexpr size_t kPiece = (size_t)1 << 20;
 constexpr int kThreads = 8, kSlots = 2;
-// a piece for each thread: below, starting the threads costs what they save
-// (4.7 MB 270 us plain, 285 so; 9.2 MB 500 / 470; 15.9 MB 840 / 650)
-constexpr size_t kSplitBytes = kThreads * kPiece;
+constexpr size_t kLeastSplit = (size_t)12 << 20;  // see split_bytes
 constexpr size_t kPinnedBytes = kThreads * kSlots * kPiece, kHugePage = (size_t)2 << 20;
 // The buffers cost 1.8 ms, 3.6 the first time, to make and give back (16 MB of huge
 // pages; 10 ms by cudaHostAlloc).  A copy of 64 MB saves that by itself (up
@@ -42,6 +41,24 @@ std::mutex g_use_mu;    // one transfer at a time
 void *g_mapped = nullptr;  // the buffers' mapping
 char *g_pinned = nullptr;  // the buffers: kThreads x kSlots pieces
 size_t g_plain = 0;     // bytes that went the plain way for want of the buffers
+
+// Cores this process may run on.
+int usable_cores() {
+    cpu_set_t set;
+    if (sched_getaffinity(0, sizeof(set), &set) == 0) return CPU_COUNT(&set);
+    return (int)std::thread::hardware_concurrency();
+}
+// The size from which a copy is split.  From three cores on 12 MB, below which
+// starting the threads costs what they save; on two, where they only share the
+// copying that one thread does, 128 MB; on one never.  Microseconds plain / split,
+// up and then down, on a B200 host: 16 cores 9 MB 471 / 473, 485 / 491, 16 MB 829 /
+// 670, 830 / 648; 3 cores 16 MB 809 / 753, 781 / 793, 24 MB 1246 / 1048, 1159 / 1081;
+// 2 cores 24 MB 1204 / 1343, 1159 / 1303, 96 MB 8304 / 5648, 4548 / 5224, 192 MB
+// 16627 / 11339, 9132 / 9577; 1 core 192 MB 17053 / 16090, 9774 / 16528.
+size_t split_bytes() {
+    const int cores = usable_cores();
+    return cores >= 3 ? kLeastSplit : cores == 2 ? (size_t)128 << 20 : SIZE_MAX;
+}
 
 bool pageable(const void *host) {
     cudaPointerAttributes a;
@@ -96,8 +113,7 @@ cudaError_t worker(int k, int threads, char *dev, char *host, size_t bytes, int 
 }
 
 cudaError_t split_copy(char *dev, char *host, size_t bytes, int device, cudaStream_t st, bool to_device) {
-    const int threads = (int)std::min<size_t>(
-        {(size_t)kThreads, std::max(1u, std::thread::hardware_concurrency() / 2), (bytes + kPiece - 1) / kPiece});
+    const int threads = (int)std::min<size_t>(kThreads, (bytes + kPiece - 1) / kPiece);
     std::atomic<int> failed{0};
     cudaError_t err[kThreads];
     std::thread pool[kThreads];
@@ -161,7 +177,7 @@ bool take_buffers(size_t bytes) {
 }
 
 cudaError_t copy(char *dev, char *host, size_t bytes, int device, cudaStream_t st, bool to_device) {
-    if (bytes >= kSplitBytes && pageable(host)) {
+    if (bytes >= kLeastSplit && bytes >= split_bytes() && pageable(host)) {
         std::unique_lock<std::mutex> use(g_use_mu, std::try_to_lock);
         if (use.owns_lock() && take_buffers(bytes)) return split_copy(dev, host, bytes, device, st, to_device);
     }

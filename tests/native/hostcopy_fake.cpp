@@ -1,5 +1,6 @@
 // The host side of the field copies (hostcopy.cu) on a fake CUDA runtime whose
-// copies are memcpy.  argv: hardware threads, then one step after another:
+// copies are memcpy.  argv: the cores that the process may use (-n: n in the machine,
+// and no affinity mask to be had), then one step after another:
 //   up N | down N    a copy of N bytes, checked; prints the number of transfers it took
 //   fail             the third and every later thread of the copies that follow finds no memory
 //   hold | drop      a holder comes or goes; drop prints the bytes pinned after it
@@ -9,6 +10,7 @@
 #include <cstdio>
 #include <cstdlib>
 #include <new>
+#include <sched.h>
 #include <string>
 #include <vector>
 
@@ -20,11 +22,17 @@ struct Region {
 };
 static Region g_regions[16];  // no allocation of the fake's own
 static int g_pins = 0;
-static unsigned g_hw = 1;
+static int g_cores = 1;
 static bool g_fail = false;         // of the main thread, which makes the threads
 static thread_local int g_left = -1;  // allocations until the first that fails; below 0: none does
 
-unsigned int std::thread::hardware_concurrency() noexcept { return g_hw; }
+unsigned int std::thread::hardware_concurrency() noexcept { return (unsigned)abs(g_cores); }
+extern "C" int sched_getaffinity(pid_t, size_t n, cpu_set_t *set) noexcept {
+    if (g_cores < 0) return -1;
+    memset(set, 0, n);
+    for (int k = 0; k < g_cores; k++) CPU_SET_S(k, n, set);
+    return 0;
+}
 
 void *operator new(size_t n) {
     if (g_left == 0) throw std::bad_alloc();
@@ -90,7 +98,7 @@ cudaError_t cudaHostUnregister(void *p) { return unpin(p); }
 }
 
 int main(int argc, char **argv) {
-    g_hw = (unsigned)atoi(argv[1]);
+    g_cores = atoi(argv[1]);
     std::vector<char> dev, host;
     for (int i = 2; i < argc; i++) {
         const std::string s = argv[i];

@@ -56,3 +56,16 @@ def test_buffers_come_after_enough_small_copies(fake):
     assert fake("hold", *seven, "drop") == before + after + [[0]]
     part = ["hold", *seven[:12], "drop"]
     assert fake(*part, *part) == ([[1]] * 6 + [[0]]) * 2
+
+
+@pytest.mark.parametrize("cores, least", [(1, None), (2, 128 * MB), (3, 12 * MB), (16, 12 * MB), (-2, 128 * MB),
+                                          (-8, 12 * MB), (0, None)])
+def test_few_cores_copy_plainly(fake, cores, least):
+    # one transfer each just below the size from which copies are split and, where
+    # they never are, of 400 MB; with the buffers there, a transfer per MB from it on
+    make = ["hold"] + ["up", 400 * MB] * 2
+    if least is None:
+        assert fake(*make, "pinned", cores=cores) == [[1], [1], [0, 0]]
+    else:
+        out = fake(*make, "up", least - 1, "down", least - 1, "up", least, "down", least, cores=cores)
+        assert out == [[400], [400], [1], [1], [least // MB], [least // MB]]
