@@ -6,6 +6,7 @@
 
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cmath>
 #include <cstdio>
 #include <cstring>
@@ -27,8 +28,6 @@ struct glac_ctx {
     double *partial4 = nullptr;  // SuperSampler partials, 4 per block (allocated on first use)
     double *obs_dev = nullptr;
     size_t obs_cap = 0;  // doubles in obs_dev
-    double *flow_partial = nullptr;  // partial sums of a flow's measurements (first measured flow)
-    size_t flow_partial_cap = 0;     // doubles
     unsigned long long *acc_dev = nullptr;
     double *staging = nullptr;
     double *scalar_dev = nullptr;
@@ -39,7 +38,7 @@ struct glac_ctx {
     uint32_t *net_pack = nullptr;
     float *esj_grid = nullptr;    // 64 floats
     Proposal prop;                // prop.net null: the fixed spread su3_eps
-    void *clover = nullptr;       // clover parts of the measurement fused into flow stage 0 (first use)
+    void *clover = nullptr;       // clover parts of the measurement fused into flow stage 0, then its partial sums (first use)
     int fused_measure = 1;        // measure inside flow stage 0 where the lattice allows it (2: 128-register cap)
     bool fused_combine = true;    // that measurement's reduction inside stage 1 where the lattice allows it
     bool has_field = false;
@@ -139,10 +138,6 @@ template <typename T> CloverParts<T> clover_view(glac_ctx *c) {
 bool fused_measure_usable(glac_ctx *c) {
     return c->fused_measure != 0 && clover_offsets_fit(c->g.V, c->d.precision == GLAC_FP64);
 }
-void ensure_clover(glac_ctx *c) {
-    if (!c->clover) ck(cudaMalloc(&c->clover, clover_bytes(c->d, c->g)), "cudaMalloc clover parts");
-}
-
 void reunit(glac_ctx *c) {
     if (c->d.precision == GLAC_FP64) launch_reunitarize(c->g, f64(c, c->cur), c->stream);
     else launch_reunitarize(c->g, f32(c, c->cur), c->stream);
@@ -165,13 +160,16 @@ struct FlowMode {
 // 12^3 x 24 57 / 60, 14^3 x 28 108 / 101; FP64 8^3 x 16 31 / 36, 10^3 x 20
 // 74 / 74, 12^3 x 24 125 / 120.
 constexpr int kSplitMaxSitesFp32 = 148 * 24 * 32 * 3 / 2 / 4, kSplitMaxSitesFp64 = 148 * 16 * 32 / 4;
+bool split_size(const glac_ctx *c) {
+    return c->g.V <= (c->d.precision == GLAC_FP32 ? kSplitMaxSitesFp32 : kSplitMaxSitesFp64);
+}
+int split_nb(const glac_ctx *c) { return c->g.Vh / c->g.N[3] / 32; }
 FlowMode flow_mode(const glac_ctx *c) {
     FlowMode m;
     const int fused_default = c->d.precision == GLAC_FP32 ? 2 : 1;
-    m.split = c->g.V <= (c->d.precision == GLAC_FP32 ? kSplitMaxSitesFp32 : kSplitMaxSitesFp64) &&
-              c->d.exp_func == GLAC_EXP_MORNINGSTAR && c->tune[FAM_FLOW] == 0 && c->fused_measure == fused_default;
+    m.split = split_size(c) && c->d.exp_func == GLAC_EXP_MORNINGSTAR && c->tune[FAM_FLOW] == 0 && c->fused_measure == fused_default;
     m.in_stage1 = c->fused_combine && (m.split ? flow_split_combines(c->g) : obs_combine_in_stage1(c->g, c->plan));
-    m.nb = m.split && m.in_stage1 ? c->g.Vh / c->g.N[3] / 32 : c->plan.nb;
+    m.nb = m.split && m.in_stage1 ? split_nb(c) : c->plan.nb;
     m.row = (size_t)6 * m.nb * c->g.N[3];
     return m;
 }
@@ -200,20 +198,26 @@ void measure_into(glac_ctx *c, double *dev_out) {
     c->launches += 3;
 }
 
-// Room for the partial sums of as many measurements as 16 MB hold (at least one,
-// at most 256), made once, whatever the length of the flow; returns how many.
-int ensure_flow_partial(glac_ctx *c, size_t row) {
-    size_t rows = ((size_t)16 << 20) / (row * sizeof(double));
-    rows = rows < 1 ? 1 : rows > 256 ? 256 : rows;
-    const size_t n = rows * row;
-    if (c->flow_partial_cap < n) {
-        if (c->flow_partial) cudaFree(c->flow_partial);
-        c->flow_partial = nullptr;
-        c->flow_partial_cap = 0;
-        ck(cudaMalloc(&c->flow_partial, n * sizeof(double)), "cudaMalloc flow partials");
-        c->flow_partial_cap = n;
+// Behind the clover parts lie the partial sums of as many measurements as 16 MB
+// hold, at least one and at most 256.
+size_t partial_rows(size_t row) {
+    const size_t rows = ((size_t)16 << 20) / (row * sizeof(double));
+    return rows < 1 ? 1 : rows > 256 ? 256 : rows;
+}
+size_t partial_offset(const glac_ctx *c) { return (clover_bytes(c->d, c->g) + 255) / 256 * 256; }
+double *flow_partial(const glac_ctx *c) {
+    return reinterpret_cast<double *>(static_cast<char *>(c->clover) + partial_offset(c));
+}
+// One allocation for both, with room for either size of a measurement's sums.
+void ensure_clover(glac_ctx *c) {
+    if (c->clover) return;
+    const size_t row = (size_t)6 * c->plan.nb * c->g.N[3];
+    size_t sums = partial_rows(row) * row;
+    if (split_size(c) && flow_split_combines(c->g)) {
+        const size_t small = (size_t)6 * split_nb(c) * c->g.N[3];
+        sums = std::max(sums, partial_rows(small) * small);
     }
-    return (int)rows;
+    ck(cudaMalloc(&c->clover, partial_offset(c) + sums * sizeof(double)), "cudaMalloc clover parts");
 }
 
 // One Luscher RK3 step: three fused stages, cur -> other -> cur -> other.
@@ -231,10 +235,7 @@ void flow_step_t(glac_ctx *c, const FlowMode &mode, cudaEvent_t *ev, double *par
     int e = 1;
     const ForceField<T> z = force_field<T>(c);
     CloverParts<T> cp;
-    if (partial) {
-        ensure_clover(c);
-        cp = clover_view<T>(c);
-    }
+    if (partial) cp = clover_view<T>(c);
     for (int stage = 0; stage < 3; stage++) {
         const int src = c->cur, dst = c->cur ^ 1;
         const LinkField<T> in = link_field<T>(c, src), out = link_field<T>(c, dst);
@@ -353,7 +354,6 @@ void glac_destroy(glac_ctx *c) {
     if (c->force) cudaFree(c->force);
     if (c->partial) cudaFree(c->partial);
     if (c->partial4) cudaFree(c->partial4);
-    if (c->flow_partial) cudaFree(c->flow_partial);
     if (c->obs_dev) cudaFree(c->obs_dev);
     if (c->acc_dev) cudaFree(c->acc_dev);
     if (c->staging) cudaFree(c->staging);
@@ -650,13 +650,16 @@ glac_status glac_flow(glac_ctx *c, int n_steps, double *obs) {
         if (obs) {
             ensure_obs(c, per * (size_t)(n_steps + 1));
             if (!fused || n_steps == 0) measure_into(c, c->obs_dev);
-            if (fused && n_steps > 0) rows = ensure_flow_partial(c, mode.row);
+            if (fused && n_steps > 0) {
+                ensure_clover(c);
+                rows = (int)partial_rows(mode.row);
+            }
         }
         for (int i = 0; i < n_steps; i++) {
             const int r = i % rows;
-            flow_step(c, mode, nullptr, fused ? c->flow_partial + mode.row * (size_t)r : nullptr);
+            flow_step(c, mode, nullptr, fused ? flow_partial(c) + mode.row * (size_t)r : nullptr);
             if (fused && (r == rows - 1 || i == n_steps - 1)) {
-                launch_obs_finalize(c->g, mode.nb, r + 1, c->flow_partial, c->obs_dev + per * (size_t)(i - r),
+                launch_obs_finalize(c->g, mode.nb, r + 1, flow_partial(c), c->obs_dev + per * (size_t)(i - r),
                                     c->stream);
                 ck_launch("measurement reduction");
                 c->launches += 1;
@@ -709,12 +712,12 @@ glac_status glac_flow_stage_times_measured(glac_ctx *c, int n_steps, double *sec
             return GLAC_ERR_STATE;
         }
         const FlowMode mode = flow_mode(c);
-        ensure_flow_partial(c, mode.row);
+        ensure_clover(c);
         cudaEvent_t ev[5];
         for (int i = 0; i < 5; i++) ck(cudaEventCreate(&ev[i]), "event create");
         double acc[4] = {0, 0, 0, 0};
         for (int k = 0; k < n_steps; k++) {
-            flow_step(c, mode, ev, c->flow_partial);
+            flow_step(c, mode, ev, flow_partial(c));
             ck(cudaEventSynchronize(ev[4]), "event sync");
             for (int i = 0; i < 4; i++) {
                 float ms = 0.f;
@@ -770,8 +773,8 @@ glac_status glac_autotune(glac_ctx *c, int reps, double *report) {
                         if (fam == FAM_FLOW) {
                             const FlowMode mode = flow_mode(c);
                             if (fused_measure_usable(c)) {
-                                ensure_flow_partial(c, mode.row);
-                                flow_step(c, mode, nullptr, c->flow_partial);
+                                ensure_clover(c);
+                                flow_step(c, mode, nullptr, flow_partial(c));
                             } else flow_step(c, mode);
                         } else if (fam == FAM_METRO) {
                             for (int k = 0; k < 8; k++) {

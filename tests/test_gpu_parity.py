@@ -578,6 +578,29 @@ def test_long_measured_flows(g, prec, N, variant, steps):
         assert np.array_equal(A.get_links(), B.get_links())
 
 
+@pytest.mark.parametrize("prec", ["fp64", "fp32"])
+def test_flow_forms_share_a_context(g, prec):
+    # a context's partial sums have one place, whichever form a flow takes and in
+    # whatever order: several warps to a link (whole and separate combination), a thread per link
+    N = (8, 8, 8, 16)
+    forms = [(0, 1), (1, 1), (0, 0), (1, 0)]
+
+    def flow(L, form):
+        L.tuning = [form[0], 0, 0]
+        L.set_option("fused_combine", form[1])
+        L.hot_start(4)
+        return L.flow(260)
+
+    want = []
+    for form in forms:
+        with lattice(g, N, prec, seed=6) as L:
+            want.append(flow(L, form))
+    for order in (forms, forms[::-1]):
+        with lattice(g, N, prec, seed=6) as L:
+            for form in order:
+                assert np.array_equal(flow(L, form), want[forms.index(form)]), form
+
+
 def test_observables_at_the_largest_time_extent(g, oracle):
     # Nt = 1024 fills the per-slice arrays of the reduction; larger Nt is rejected at creation
     N = (4, 4, 4, 1024)
