@@ -301,8 +301,16 @@ void launch_flow_stage(const Geom &g, const LinkField<T> &in, const LinkField<T>
         else flow_dispatch<T, 0, 2>(regs, shape, st, g, in, out, zf, a, b);
         return;
     }
-#define GLAC_FLOW_CASE(K, S) \
-    if (kind == K && stage == S) { launch_chained(k_flow_stage<T, K, S, 0>, grid.x, 128, st, g, in, out, zf, a, b); return; }
+    // The other exponentials: in FP64 at 128 registers too (stage 2 of 24^3 x 48 on B200,
+    // capped / uncapped: Luscher 510 / 721 us, second order 436 / 530), but the fourth
+    // order, which spills 108 B so (508 / 477); in FP32 uncapped.
+#define GLAC_FLOW_CASE(K, S)                                                                                  \
+    if (kind == K && stage == S) {                                                                            \
+        if constexpr (sizeof(T) == 8 && K != EXP_TAYLOR4)                                                     \
+            launch_chained(k_flow_stage_r128<T, K, S, 0>, grid.x, 128, st, g, in, out, zf, a, b);              \
+        else launch_chained(k_flow_stage<T, K, S, 0>, grid.x, 128, st, g, in, out, zf, a, b);                  \
+        return;                                                                                               \
+    }
     GLAC_FLOW_CASE(1, 0) GLAC_FLOW_CASE(1, 1) GLAC_FLOW_CASE(1, 2)
     GLAC_FLOW_CASE(2, 0) GLAC_FLOW_CASE(2, 1) GLAC_FLOW_CASE(2, 2)
     GLAC_FLOW_CASE(3, 0) GLAC_FLOW_CASE(3, 1) GLAC_FLOW_CASE(3, 2)
