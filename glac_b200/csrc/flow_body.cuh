@@ -18,7 +18,6 @@ template <typename T> __device__ __forceinline__ AH8<T> flow_force(const M3<T> &
 template <typename T, int KIND, int STAGE>
 __device__ __forceinline__ void flow_update(const M3<T> &U, const AH8<T> &Z, const LinkField<T> &out,
                                             const ForceField<T> &zf, T alpha, T beta, int mu, int p, int s) {
-    chain_release();
     AH8<T> M;
     if (STAGE == 0) {
         M = ah_scale(alpha, Z);
@@ -28,6 +27,7 @@ __device__ __forceinline__ void flow_update(const M3<T> &U, const AH8<T> &Z, con
         M = ah_axpby(alpha, Z, beta, W);
         if (STAGE == 1) zf.store(mu, p, s, M);
     }
+    chain_release();
     if (KIND == EXP_MORNINGSTAR) {
         // U' = U + (exp(M) - 1) U: the small product first, one rounding at |U|
         out.store(mu, p, s, mul_plus_right(expm_morningstar<T, true>(M), U));
