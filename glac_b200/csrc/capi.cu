@@ -3,6 +3,7 @@
 #include "../../include/glac_b200.h"
 #include "hostcopy.cuh"
 #include "kernels.cuh"
+#include "variants.cuh"
 
 #include <cuda_runtime.h>
 
@@ -253,7 +254,7 @@ void flow_step_t(glac_ctx *c, const FlowMode &mode, cudaEvent_t *ev, double *par
         } else if (stage == 1 && partial && mode.in_stage1) {
             // the site-per-thread stage where the flow family's chosen variant has that shape
             launch_flow_stage1_combine(c->g, in, out, z, c->d.exp_func, alpha[1], beta[1], cp, c->plan, partial,
-                                       variant_shape(FAM_FLOW, sizeof(T) == 4, c->tune[FAM_FLOW]) == 3, c->stream);
+                                       variant_form(FAM_FLOW, sizeof(T) == 4, c->tune[FAM_FLOW]).shape == 3, c->stream);
         } else {
             launch_flow_stage(c->g, in, out, z, stage, c->d.exp_func, alpha[stage], beta[stage], c->tune[FAM_FLOW],
                               c->stream);

@@ -15,6 +15,7 @@
 #include "../../include/glac_b200.h"
 #include "hostcopy.cuh"
 #include "kernels.cuh"
+#include "variants.cuh"
 
 #include <cuda_runtime.h>
 
@@ -210,7 +211,7 @@ template <typename T> void flow_t(glac_ensemble *E, int n, bool measure) {
     const double alpha[3] = {eps * 0.25, eps * 0.8888888888888888, 0.75 * eps};
     const double bet[3] = {0.0, -(eps * 0.4722222222222222), -1.0};
     const bool fp32 = sizeof(T) == 4;
-    const int phase = variant_shape(FAM_FLOW, fp32, E->tune[FAM_FLOW]) == 1 ? ENS_FLOW1 : ENS_FLOW0;
+    const int phase = variant_form(FAM_FLOW, fp32, E->tune[FAM_FLOW]).shape == 1 ? ENS_FLOW1 : ENS_FLOW0;
     int cur = 1;
     // the measurement after step k inside stage 0 of step k + 1 (the field that
     // stage flows is the one to measure), the last one in a pass of its own

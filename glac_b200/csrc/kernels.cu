@@ -6,6 +6,7 @@
 #include "launch.cuh"
 #include "metropolis.cuh"
 #include "learned.cuh"
+#include "variants.cuh"
 
 #include <algorithm>
 #include <stdexcept>
@@ -219,73 +220,21 @@ GLAC_FLOW_KERNEL(k_flow_stage_r128, __maxnreg__(128))
 GLAC_FLOW_KERNEL(k_flow_stage_r80, __maxnreg__(80))
 GLAC_FLOW_KERNEL(k_flow_stage_r96, __maxnreg__(96))
 
-// Launch-bound variants (minimum resident blocks of 128 threads per SM, i.e.
-// the register cap) that the autotuner chooses among; variant 0 is the default.
-// Register caps per variant ([fp64, fp32]; 0 = no cap, -1 = unused slot); the
-// flow family also varies the site-block shape.  The flow stage waits on its
-// neighbour links (L2 hits), so resident warps count for more than registers:
-// its default caps give 16 (FP64) and 24 (FP32) warps per SM.  Stage 2 on B200,
-// capped / uncapped: FP64 24^3 x 48 427 / 528 us, 16^3 x 32 97 / 114; FP32
-// 32^3 x 64 662 / 700, 16^3 x 32 51 / 53.  Metropolis: see metro_regs.
-const int kFlowRegs[2][kMaxVariants] = {{128, 0, 0, 128}, {80, 0, 0, 96}};
-const int kFlowShape[2][kMaxVariants] = {{0, 0, 1, 2}, {0, 0, 3, 0}};
-const int kMetroRegs[2][kMaxVariants] = {{0, 128, -1, -1}, {96, 0, 80, 128}};
-const int kObsRegs[2][kMaxVariants] = {{0, 128, -1, -1}, {0, 128, 168, -1}};
-
-int num_variants(Family f, bool fp32) {
-    const int(*t)[kMaxVariants] = f == FAM_FLOW ? kFlowRegs : f == FAM_METRO ? kMetroRegs : kObsRegs;
-    int n = 0;
-    while (n < kMaxVariants && t[fp32 ? 1 : 0][n] >= 0) n++;
-    return n;
-}
-int variant_regs(Family f, bool fp32, int v) {
-    const int(*t)[kMaxVariants] = f == FAM_FLOW ? kFlowRegs : f == FAM_METRO ? kMetroRegs : kObsRegs;
-    return (v >= 0 && v < kMaxVariants) ? t[fp32 ? 1 : 0][v] : 0;
-}
-
-int variant_shape(Family f, bool fp32, int v) {
-    return (f == FAM_FLOW && v >= 0 && v < kMaxVariants) ? kFlowShape[fp32 ? 1 : 0][v] : 0;
-}
-
-template <typename T, int KIND, int STAGE, int SHAPE>
-static void flow_dispatch_caps(int regs, cudaStream_t st, const Geom &g, const LinkField<T> &in,
-                               const LinkField<T> &out, const ForceField<T> &zf, T a, T b) {
-    const dim3 grid(8 * ((g.Vh + 127) / 128));
-    switch (regs) {
-    case 128: launch_chained(k_flow_stage_r128<T, KIND, STAGE, SHAPE>, grid.x, 128, st, g, in, out, zf, a, b); break;
-    case 96:
-        if constexpr (sizeof(T) == 4) {
-            launch_chained(k_flow_stage_r96<T, KIND, STAGE, SHAPE>, grid.x, 128, st, g, in, out, zf, a, b);
-            break;
-        }
-        [[fallthrough]];
-    case 80:
-        if constexpr (sizeof(T) == 4) {
-            launch_chained(k_flow_stage_r80<T, KIND, STAGE, SHAPE>, grid.x, 128, st, g, in, out, zf, a, b);
-            break;
-        }
-        [[fallthrough]];  // no 80-register FP64 variant
-    default: launch_chained(k_flow_stage<T, KIND, STAGE, SHAPE>, grid.x, 128, st, g, in, out, zf, a, b); break;
-    }
-}
-
 template <typename T, int KIND, int STAGE>
-static void flow_dispatch(int regs, int shape, cudaStream_t st, const Geom &g, const LinkField<T> &in,
+static void flow_dispatch(VariantForm form, cudaStream_t st, const Geom &g, const LinkField<T> &in,
                           const LinkField<T> &out, const ForceField<T> &zf, T a, T b) {
+    const unsigned grid = 8 * ((g.Vh + 127) / 128);
     if constexpr (sizeof(T) == 4) {
-        if (shape == 3) {
-            const dim3 grid(2 * ((g.Vh + kSiteBlock - 1) / kSiteBlock));
-            launch_chained(k_flow_stage_site<T, KIND, STAGE>, grid.x, kSiteBlock, st, g, in, out, zf, a, b);
-            return;
-        }
+        if (form.shape == 3)
+            launch_chained(k_flow_stage_site<T, KIND, STAGE>, 2 * ((g.Vh + kSiteBlock - 1) / kSiteBlock), kSiteBlock, st,
+                           g, in, out, zf, a, b);
+        else if (form.regs == 96) launch_chained(k_flow_stage_r96<T, KIND, STAGE, 0>, grid, 128, st, g, in, out, zf, a, b);
+        else launch_chained(k_flow_stage_r80<T, KIND, STAGE, 0>, grid, 128, st, g, in, out, zf, a, b);
+    } else {
+        if (form.shape == 1) launch_chained(k_flow_stage<T, KIND, STAGE, 1>, (g.Vh + 15) / 16, 128, st, g, in, out, zf, a, b);
+        else if (form.shape == 2) launch_chained(k_flow_stage_r128<T, KIND, STAGE, 2>, grid, 128, st, g, in, out, zf, a, b);
+        else launch_chained(k_flow_stage_r128<T, KIND, STAGE, 0>, grid, 128, st, g, in, out, zf, a, b);
     }
-    if (shape == 1) {
-        const dim3 grid((g.Vh + 15) / 16);
-        launch_chained(k_flow_stage<T, KIND, STAGE, 1>, grid.x, 128, st, g, in, out, zf, a, b);
-        return;
-    }
-    if (shape == 2) flow_dispatch_caps<T, KIND, STAGE, 2>(regs, st, g, in, out, zf, a, b);
-    else flow_dispatch_caps<T, KIND, STAGE, 0>(regs, st, g, in, out, zf, a, b);
 }
 
 template <typename T>
@@ -293,12 +242,11 @@ void launch_flow_stage(const Geom &g, const LinkField<T> &in, const LinkField<T>
                        int stage, int kind, double alpha, double beta, int variant, cudaStream_t st) {
     const dim3 grid(8 * ((g.Vh + 127) / 128));
     const T a = (T)alpha, b = (T)beta;
-    const bool fp32 = sizeof(T) == 4;
     if (kind == EXP_MORNINGSTAR) {
-        const int regs = variant_regs(FAM_FLOW, fp32, variant), shape = variant_shape(FAM_FLOW, fp32, variant);
-        if (stage == 0) flow_dispatch<T, 0, 0>(regs, shape, st, g, in, out, zf, a, b);
-        else if (stage == 1) flow_dispatch<T, 0, 1>(regs, shape, st, g, in, out, zf, a, b);
-        else flow_dispatch<T, 0, 2>(regs, shape, st, g, in, out, zf, a, b);
+        const VariantForm form = variant_form(FAM_FLOW, sizeof(T) == 4, variant);
+        if (stage == 0) flow_dispatch<T, 0, 0>(form, st, g, in, out, zf, a, b);
+        else if (stage == 1) flow_dispatch<T, 0, 1>(form, st, g, in, out, zf, a, b);
+        else flow_dispatch<T, 0, 2>(form, st, g, in, out, zf, a, b);
         return;
     }
     // The other exponentials: in FP64 at 128 registers too (stage 2 of 24^3 x 48 on B200,
@@ -579,42 +527,31 @@ GLAC_METRO_KERNEL(k_metropolis_r80, __maxnreg__(80))
 #undef GLAC_METRO_KERNEL
 
 template <typename T, bool LEARNED>
-static void metro_dispatch(int regs, dim3 grid, cudaStream_t st, const Geom &g, const LinkField<T> &L, int mu,
+static void metro_dispatch(int regs, unsigned grid, cudaStream_t st, const Geom &g, const LinkField<T> &L, int mu,
                            int p, T mfac, T e, T sq, int nhits, uint32_t k0, uint32_t k1, uint32_t sweep,
                            uint32_t stream_id, unsigned long long *acc, const Proposal &P, float beta) {
-    switch (regs) {
-    case 128: launch_chained(k_metropolis_r128<T, LEARNED>, grid.x, 128, st, g, L, mu, p, mfac, e, sq, nhits, k0, k1, sweep, stream_id, acc, P, beta); break;
-    case 96: launch_chained(k_metropolis_r96<T, LEARNED>, grid.x, 128, st, g, L, mu, p, mfac, e, sq, nhits, k0, k1, sweep, stream_id, acc, P, beta); break;
-    case 80: launch_chained(k_metropolis_r80<T, LEARNED>, grid.x, 128, st, g, L, mu, p, mfac, e, sq, nhits, k0, k1, sweep, stream_id, acc, P, beta); break;
-    default: launch_chained(k_metropolis<T, LEARNED>, grid.x, 128, st, g, L, mu, p, mfac, e, sq, nhits, k0, k1, sweep, stream_id, acc, P, beta); break;
-    }
-}
-
-// Register cap of a sub-sweep.  FP32's default is 96 (five blocks per SM), but
-// 128 (four) where a fifth block finds no work, up to one wave of blocks, and for
-// the learned spread, whose kernel spills at 96.  Microseconds per sweep on B200
-// at 128 / 96: 12^3 x 24 112 / 115, 24^3 x 48 788 / 778, 32^3 x 64 2276 / 2248;
-// learned 24^3 x 48 898 / 934 (uncapped 930).  FP64's default is uncapped (three
-// blocks per SM), but 128 with a small spill from ten blocks per SM on: 16^3 x 32
-// 347 / 331 us, 24^3 x 48 1463 / 1498, 32^3 x 64 4310 / 4432.
-static int metro_regs(bool fp32, int variant, bool learned, int blocks) {
-    if (fp32 && variant == 0 && (learned || blocks <= 5 * 148)) return 128;
-    if (!fp32 && variant == 0 && blocks > 10 * 148) return 128;
-    return variant_regs(FAM_METRO, fp32, variant);
+    auto launch = [&](auto kernel) {
+        launch_chained(kernel, grid, 128, st, g, L, mu, p, mfac, e, sq, nhits, k0, k1, sweep, stream_id, acc, P, beta);
+    };
+    if (regs == 128) launch(k_metropolis_r128<T, LEARNED>);
+    else if constexpr (sizeof(T) == 8) launch(k_metropolis<T, LEARNED>);
+    else if (regs == 96) launch(k_metropolis_r96<T, LEARNED>);
+    else launch(k_metropolis_r80<T, LEARNED>);
 }
 
 template <typename T>
 void launch_metropolis(const Geom &g, const LinkField<T> &L, int mu, int p, double beta, double eps, int nhits,
                        uint64_t seed, uint32_t sweep, uint32_t stream_id, unsigned long long *acc, int variant,
                        const Proposal &P, cudaStream_t st) {
-    const dim3 grid((g.Vh + 127) / 128);  // 128 threads: the learned path's shared memory holds 4 warps
+    const unsigned grid = (g.Vh + 127) / 128;  // 128 threads: the learned path's shared memory holds 4 warps
     const T mfac = (T)(-beta / 3.0), e = (T)eps, sq = (T)sqrt(1.0 - eps * eps);
     const uint32_t k0 = (uint32_t)seed, k1 = (uint32_t)(seed >> 32);
     if (variant == 0 && metropolis_splits(g)) {
         launch_metropolis_split(g, L, mu, p, mfac, e, sq, nhits, k0, k1, sweep, stream_id, acc, P, (float)beta, st);
         return;
     }
-    const int regs = metro_regs(sizeof(T) == 4, variant, P.net != nullptr, (int)grid.x);
+    const int regs = variant == 0 ? metro_default_regs(sizeof(T) == 4, P.net != nullptr, (int)grid)
+                                  : variant_form(FAM_METRO, sizeof(T) == 4, variant).regs;
     if (P.net)
         metro_dispatch<T, true>(regs, grid, st, g, L, mu, p, mfac, e, sq, nhits, k0, k1, sweep, stream_id, acc, P,
                                 (float)beta);
@@ -1387,12 +1324,14 @@ void launch_ens_metropolis(const LatSlot<T> *slots, const int *start, int nblock
                            bool flips, int variant, cudaStream_t st) {
     const T e = (T)eps, sq = (T)sqrt(1.0 - eps * eps);
     const uint32_t k0 = (uint32_t)seed, k1 = (uint32_t)(seed >> 32);
-    switch (variant_regs(FAM_METRO, sizeof(T) == 4, variant)) {
-    case 128: kb_metropolis_r128<T><<<nblocks, 128, 0, st>>>(slots, start, M, fsel, mu, p, e, sq, nhits, k0, k1, sweep_base, sweep_off, flips); break;
-    case 96: kb_metropolis_r96<T><<<nblocks, 128, 0, st>>>(slots, start, M, fsel, mu, p, e, sq, nhits, k0, k1, sweep_base, sweep_off, flips); break;
-    case 80: kb_metropolis_r80<T><<<nblocks, 128, 0, st>>>(slots, start, M, fsel, mu, p, e, sq, nhits, k0, k1, sweep_base, sweep_off, flips); break;
-    default: kb_metropolis<T><<<nblocks, 128, 0, st>>>(slots, start, M, fsel, mu, p, e, sq, nhits, k0, k1, sweep_base, sweep_off, flips); break;
-    }
+    auto launch = [&](auto kernel) {
+        kernel<<<nblocks, 128, 0, st>>>(slots, start, M, fsel, mu, p, e, sq, nhits, k0, k1, sweep_base, sweep_off, flips);
+    };
+    const int regs = variant_form(FAM_METRO, sizeof(T) == 4, variant).regs;
+    if (regs == 128) launch(kb_metropolis_r128<T>);
+    else if constexpr (sizeof(T) == 8) launch(kb_metropolis<T>);
+    else if (regs == 96) launch(kb_metropolis_r96<T>);
+    else launch(kb_metropolis_r80<T>);
 }
 
 #define GLAC_ENS_FLOW_KERNEL(NAME, ATTR)                                                                     \
@@ -1410,49 +1349,31 @@ GLAC_ENS_FLOW_KERNEL(kb_flow_stage_r96, __maxnreg__(96))
 GLAC_ENS_FLOW_KERNEL(kb_flow_stage_r128, __maxnreg__(128))
 #undef GLAC_ENS_FLOW_KERNEL
 
-template <typename T, int STAGE, int SHAPE>
-static void ens_flow_dispatch_caps(int regs, int nblocks, cudaStream_t st, const LatSlot<T> *slots,
-                                   const int *start, int M, int src, int dst, T a, T b) {
-    switch (regs) {
-    case 128: kb_flow_stage_r128<T, STAGE, SHAPE><<<nblocks, 128, 0, st>>>(slots, start, M, src, dst, a, b); break;
-    case 96:
-        if constexpr (sizeof(T) == 4) {
-            kb_flow_stage_r96<T, STAGE, SHAPE><<<nblocks, 128, 0, st>>>(slots, start, M, src, dst, a, b);
-            break;
-        }
-        [[fallthrough]];
-    case 80:
-        if constexpr (sizeof(T) == 4) {
-            kb_flow_stage_r80<T, STAGE, SHAPE><<<nblocks, 128, 0, st>>>(slots, start, M, src, dst, a, b);
-            break;
-        }
-        [[fallthrough]];
-    default: kb_flow_stage<T, STAGE, SHAPE><<<nblocks, 128, 0, st>>>(slots, start, M, src, dst, a, b); break;
-    }
-}
-
+// shape 2 has shape 0's block table (ens_blocks, ENS_FLOW0); only the chunk order differs
 template <typename T, int STAGE>
-static void ens_flow_dispatch(int regs, int shape, int nblocks, cudaStream_t st, const LatSlot<T> *slots,
+static void ens_flow_dispatch(VariantForm form, int nblocks, cudaStream_t st, const LatSlot<T> *slots,
                               const int *start, int M, int src, int dst, T a, T b) {
-    if (shape == 1) {
-        kb_flow_stage<T, STAGE, 1><<<nblocks, 128, 0, st>>>(slots, start, M, src, dst, a, b);
-        return;
+    auto launch = [&](auto kernel) { kernel<<<nblocks, 128, 0, st>>>(slots, start, M, src, dst, a, b); };
+    if constexpr (sizeof(T) == 4) {
+        if (form.regs == 96) launch(kb_flow_stage_r96<T, STAGE, 0>);
+        else if (form.regs == 80) launch(kb_flow_stage_r80<T, STAGE, 0>);
+        else launch(kb_flow_stage<T, STAGE, 0>);
+    } else {
+        if (form.shape == 1) launch(kb_flow_stage<T, STAGE, 1>);
+        else if (form.shape == 2) launch(kb_flow_stage_r128<T, STAGE, 2>);
+        else launch(kb_flow_stage_r128<T, STAGE, 0>);
     }
-    // shape 2 has shape 0's block table (ens_blocks, ENS_FLOW0); only the chunk order differs
-    if (shape == 2) ens_flow_dispatch_caps<T, STAGE, 2>(regs, nblocks, st, slots, start, M, src, dst, a, b);
-    else ens_flow_dispatch_caps<T, STAGE, 0>(regs, nblocks, st, slots, start, M, src, dst, a, b);
 }
 
 // nblocks: the table of the variant's shape (ENS_FLOW0 or ENS_FLOW1)
 template <typename T>
 void launch_ens_flow_stage(const LatSlot<T> *slots, const int *start, int nblocks, int M, int src, int dst, int stage,
                            double alpha, double beta, int variant, cudaStream_t st) {
-    const bool fp32 = sizeof(T) == 4;
-    const int regs = variant_regs(FAM_FLOW, fp32, variant), shape = variant_shape(FAM_FLOW, fp32, variant);
+    const VariantForm form = variant_form(FAM_FLOW, sizeof(T) == 4, variant);
     const T a = (T)alpha, b = (T)beta;
-    if (stage == 0) ens_flow_dispatch<T, 0>(regs, shape, nblocks, st, slots, start, M, src, dst, a, b);
-    else if (stage == 1) ens_flow_dispatch<T, 1>(regs, shape, nblocks, st, slots, start, M, src, dst, a, b);
-    else ens_flow_dispatch<T, 2>(regs, shape, nblocks, st, slots, start, M, src, dst, a, b);
+    if (stage == 0) ens_flow_dispatch<T, 0>(form, nblocks, st, slots, start, M, src, dst, a, b);
+    else if (stage == 1) ens_flow_dispatch<T, 1>(form, nblocks, st, slots, start, M, src, dst, a, b);
+    else ens_flow_dispatch<T, 2>(form, nblocks, st, slots, start, M, src, dst, a, b);
 }
 
 #define GLAC_ENS_OBS_KERNEL(NAME, ATTR)                                                                      \
@@ -1475,16 +1396,12 @@ __global__ void kb_obs_finalize(const LatSlot<T> *__restrict__ slots, int meas) 
 template <typename T>
 void launch_ens_observables(const LatSlot<T> *slots, const int *start, int nblocks, int M, int fsel, int meas,
                             int variant, cudaStream_t st) {
-    switch (variant_regs(FAM_OBS, sizeof(T) == 4, variant)) {
-    case 128: kb_observables_r128<T><<<nblocks, 128, 0, st>>>(slots, start, M, fsel); break;
-    case 168:
-        if constexpr (sizeof(T) == 4) {
-            kb_observables_r168<T><<<nblocks, 128, 0, st>>>(slots, start, M, fsel);
-            break;
-        }
-        [[fallthrough]];  // no 168-register FP64 variant
-    default: kb_observables<T><<<nblocks, 128, 0, st>>>(slots, start, M, fsel); break;
-    }
+    const int regs = variant_form(FAM_OBS, sizeof(T) == 4, variant).regs;
+    auto launch = [&](auto kernel) { kernel<<<nblocks, 128, 0, st>>>(slots, start, M, fsel); };
+    if (regs == 128) launch(kb_observables_r128<T>);
+    else if constexpr (sizeof(T) == 8) launch(kb_observables<T>);
+    else if (regs == 168) launch(kb_observables_r168<T>);
+    else launch(kb_observables<T>);
     kb_obs_finalize<T><<<M, 1024, 0, st>>>(slots, meas);
 }
 
