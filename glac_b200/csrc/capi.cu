@@ -1,8 +1,10 @@
 // C ABI (include/glac_b200.h): contexts, device buffers, stream, and the
 // sequencing of the hot-path kernels.
 #include "../../include/glac_b200.h"
+#include "autotune.cuh"
 #include "hostcopy.cuh"
 #include "kernels.cuh"
+#include "metropolis.cuh"
 #include "variants.cuh"
 
 #include <cuda_runtime.h>
@@ -732,8 +734,8 @@ glac_status glac_flow_stage_times_measured(glac_ctx *c, int n_steps, double *sec
     });
 }
 
-// Launch-variant autotuner: times every variant of the flow-stage, Metropolis
-// and observable kernels on this context's lattice and keeps the fastest.
+// Launch-variant autotuner: times the variants of the flow-stage, Metropolis and
+// observable kernels on this context's lattice (autotune.cuh) and keeps the fastest.
 // The field, the sweep counter and the Philox stream are restored afterwards.
 // report (optional, 3 x kMaxVariants doubles) receives the mean seconds per
 // call of each variant (0 where a family has fewer variants).
@@ -749,9 +751,6 @@ glac_status glac_autotune(glac_ctx *c, int reps, double *report) {
            "backup");
         const uint32_t sweep0 = c->sweep;
         const int cur0 = c->cur;
-        cudaEvent_t e0, e1;
-        ck(cudaEventCreate(&e0), "event");
-        ck(cudaEventCreate(&e1), "event");
         auto restore = [&]() {
             c->cur = cur0;
             c->sweep = sweep0;
@@ -759,57 +758,50 @@ glac_status glac_autotune(glac_ctx *c, int reps, double *report) {
                                c->stream),
                "restore");
         };
+        // flows measure after every step where the measurement runs inside the
+        // stages, so the flow family is timed on such steps
+        if (fused_measure_usable(c)) ensure_clover(c);
+        auto call = [&](int fam, int v) {
+            c->tune[fam] = v;
+            if (fam == FAM_FLOW) {
+                flow_step(c, flow_mode(c), nullptr, fused_measure_usable(c) ? flow_partial(c) : nullptr);
+            } else if (fam == FAM_METRO) {
+                for (int k = 0; k < 8; k++) {
+                    if (fp32)
+                        launch_metropolis(c->g, f32(c, c->cur), k >> 1, k & 1, c->d.beta, c->d.su3_eps, c->d.n_updates,
+                                          c->d.seed, c->sweep, c->d.stream_id, c->acc_dev, v, c->prop, c->stream);
+                    else
+                        launch_metropolis(c->g, f64(c, c->cur), k >> 1, k & 1, c->d.beta, c->d.su3_eps, c->d.n_updates,
+                                          c->d.seed, c->sweep, c->d.stream_id, c->acc_dev, v, c->prop, c->stream);
+                    ck_launch("metropolis");
+                }
+            } else measure_into(c, c->obs_dev);
+        };
+        auto alike = [&](int fam, int n, int *same) {
+            if (fam == FAM_FLOW)
+                first_alike(n, [&](int v) {
+                    c->tune[FAM_FLOW] = v;
+                    return lattice_flow_form(fp32, v, flow_mode(c).split, c->d.exp_func == GLAC_EXP_MORNINGSTAR);
+                }, same);
+            else if (fam == FAM_METRO)
+                first_alike(n, [&](int v) {
+                    return lattice_metro_form(fp32, v, metropolis_splits(c->g), c->prop.net != nullptr, (c->g.Vh + 127) / 128);
+                }, same);
+            else
+                for (int v = 0; v < n; v++) same[v] = v;
+        };
         double table[3][kMaxVariants] = {{0}};
         for (int fam = 0; fam < 3; fam++) {
-            const int nv = num_variants((Family)fam, fp32);
-            int best = 0;
-            double best_t = 1e300;
-            for (int v = 0; v < nv; v++) {
-                c->tune[fam] = v;
-                for (int pass = 0; pass < 2; pass++) {  // pass 0 warms up
-                    ck(cudaEventRecord(e0, c->stream), "event");
-                    for (int r = 0; r < reps; r++) {
-                        // flows measure after every step where the measurement runs
-                        // inside the stages, so the flow family is timed on such steps
-                        if (fam == FAM_FLOW) {
-                            const FlowMode mode = flow_mode(c);
-                            if (fused_measure_usable(c)) {
-                                ensure_clover(c);
-                                flow_step(c, mode, nullptr, flow_partial(c));
-                            } else flow_step(c, mode);
-                        } else if (fam == FAM_METRO) {
-                            for (int k = 0; k < 8; k++) {
-                                if (fp32)
-                                    launch_metropolis(c->g, f32(c, c->cur), k >> 1, k & 1, c->d.beta, c->d.su3_eps,
-                                                      c->d.n_updates, c->d.seed, c->sweep, c->d.stream_id, c->acc_dev,
-                                                      v, c->prop, c->stream);
-                                else
-                                    launch_metropolis(c->g, f64(c, c->cur), k >> 1, k & 1, c->d.beta, c->d.su3_eps,
-                                                      c->d.n_updates, c->d.seed, c->sweep, c->d.stream_id, c->acc_dev,
-                                                      v, c->prop, c->stream);
-                                ck_launch("metropolis");
-                            }
-                        } else measure_into(c, c->obs_dev);
-                    }
-                    ck(cudaEventRecord(e1, c->stream), "event");
-                    ck(cudaEventSynchronize(e1), "event sync");
-                    restore();
-                }
-                float ms = 0.f;
-                ck(cudaEventElapsedTime(&ms, e0, e1), "elapsed");
-                const double t = ms * 1e-3 / reps;
-                table[fam][v] = t;
-                if (t < best_t) { best_t = t; best = v; }
-            }
-            c->tune[fam] = best;
+            const int n = num_variants((Family)fam, fp32);
+            int same[kMaxVariants];
+            alike(fam, n, same);
+            c->tune[fam] = time_variants(n, same, reps, c->stream, [&](int v) { call(fam, v); }, restore, ck, table[fam]);
         }
         ck(cudaStreamSynchronize(c->stream), "sync");
-        cudaEventDestroy(e0);
-        cudaEventDestroy(e1);
         cudaFree(backup);
         if (report)
             for (int f = 0; f < 3; f++)
-                for (int v = 0; v < kMaxVariants; v++) report[3 * 0 + f * kMaxVariants + v] = table[f][v];
+                for (int v = 0; v < kMaxVariants; v++) report[f * kMaxVariants + v] = table[f][v];
         return GLAC_OK;
     });
 }

@@ -13,6 +13,7 @@
 // counter of the Philox streams lives in device memory, so replays draw fresh
 // numbers.
 #include "../../include/glac_b200.h"
+#include "autotune.cuh"
 #include "hostcopy.cuh"
 #include "kernels.cuh"
 #include "variants.cuh"
@@ -676,7 +677,7 @@ glac_status glac_ensemble_set_tuning(glac_ensemble *E, const int *v) {
     return GLAC_OK;
 }
 
-// Times every launch variant of the flow, Metropolis and observable families on
+// Times the launch variants of the flow, Metropolis and observable families on
 // the whole ensemble (in the flow buffers: the chain, its sweep counter and the
 // acceptance counters are left as they were) and keeps the fastest.
 // report[4 f + v] = seconds per flow step / per sweep / per measurement (0 for
@@ -692,46 +693,31 @@ glac_status glac_ensemble_autotune(glac_ensemble *E, int reps, double *report) {
                             E->stream),
             "save acc");
         double rep[12] = {0};
-        cudaEvent_t e0, e1;
-        eck(cudaEventCreate(&e0), "event");
-        eck(cudaEventCreate(&e1), "event");
+        auto restore = [&] {
+            eck(cudaMemcpyAsync(E->field[1], E->field[0], E->field_total, cudaMemcpyDeviceToDevice, E->stream), "copy");
+        };
+        restore();
         // the observable family measures the flow buffer into row 0 of each lattice's
         // rows (allocated since creation)
         for (int fam = 0; fam < 3; fam++) {
-            const int nv = num_variants((Family)fam, fp32);
-            int best = E->tune[fam];
-            double best_t = 1e30;
-            for (int v = 0; v < nv; v++) {
+            const int n = num_variants((Family)fam, fp32);
+            int same[kMaxVariants];
+            first_alike(n, [&](int v) { return variant_form((Family)fam, fp32, v); }, same);
+            auto call = [&](int v) {
                 E->tune[fam] = v;
-                for (int pass = 0; pass < 2; pass++) {  // pass 0 warms up
-                    eck(cudaMemcpyAsync(E->field[1], E->field[0], E->field_total, cudaMemcpyDeviceToDevice, E->stream),
-                        "copy");
-                    eck(cudaEventRecord(e0, E->stream), "event");
-                    for (int r = 0; r < reps; r++) {
-                        if (fam == FAM_METRO) {
-                            if (fp32) sweeps_t<float>(E, 1, 1);
-                            else sweeps_t<double>(E, 1, 1);
-                        } else if (fam == FAM_OBS) {
-                            if (fp32) observe_t<float>(E, 1, 0);
-                            else observe_t<double>(E, 1, 0);
-                        } else {
-                            if (fp32) flow_t<float>(E, 1, false);
-                            else flow_t<double>(E, 1, false);
-                        }
-                    }
-                    eck(cudaEventRecord(e1, E->stream), "event");
-                    eck(cudaEventSynchronize(e1), "sync");
+                if (fam == FAM_METRO) {
+                    if (fp32) sweeps_t<float>(E, 1, 1);
+                    else sweeps_t<double>(E, 1, 1);
+                } else if (fam == FAM_OBS) {
+                    if (fp32) observe_t<float>(E, 1, 0);
+                    else observe_t<double>(E, 1, 0);
+                } else {
+                    if (fp32) flow_t<float>(E, 1, false);
+                    else flow_t<double>(E, 1, false);
                 }
-                float ms = 0.f;
-                eck(cudaEventElapsedTime(&ms, e0, e1), "elapsed");
-                const double t = ms * 1e-3 / reps;
-                rep[4 * fam + v] = t;
-                if (t < best_t) { best_t = t; best = v; }
-            }
-            E->tune[fam] = best;
+            };
+            E->tune[fam] = time_variants(n, same, reps, E->stream, call, restore, eck, rep + 4 * fam);
         }
-        cudaEventDestroy(e0);
-        cudaEventDestroy(e1);
         eck(cudaMemcpyAsync(E->acc, acc_save.data(), E->M * sizeof(unsigned long long), cudaMemcpyHostToDevice,
                             E->stream),
             "restore acc");

@@ -546,17 +546,17 @@ void launch_metropolis(const Geom &g, const LinkField<T> &L, int mu, int p, doub
     const unsigned grid = (g.Vh + 127) / 128;  // 128 threads: the learned path's shared memory holds 4 warps
     const T mfac = (T)(-beta / 3.0), e = (T)eps, sq = (T)sqrt(1.0 - eps * eps);
     const uint32_t k0 = (uint32_t)seed, k1 = (uint32_t)(seed >> 32);
-    if (variant == 0 && metropolis_splits(g)) {
+    const VariantForm form =
+        lattice_metro_form(sizeof(T) == 4, variant, metropolis_splits(g), P.net != nullptr, (int)grid);
+    if (form == kSplitForm) {
         launch_metropolis_split(g, L, mu, p, mfac, e, sq, nhits, k0, k1, sweep, stream_id, acc, P, (float)beta, st);
         return;
     }
-    const int regs = variant == 0 ? metro_default_regs(sizeof(T) == 4, P.net != nullptr, (int)grid)
-                                  : variant_form(FAM_METRO, sizeof(T) == 4, variant).regs;
     if (P.net)
-        metro_dispatch<T, true>(regs, grid, st, g, L, mu, p, mfac, e, sq, nhits, k0, k1, sweep, stream_id, acc, P,
+        metro_dispatch<T, true>(form.regs, grid, st, g, L, mu, p, mfac, e, sq, nhits, k0, k1, sweep, stream_id, acc, P,
                                 (float)beta);
     else
-        metro_dispatch<T, false>(regs, grid, st, g, L, mu, p, mfac, e, sq, nhits, k0, k1, sweep, stream_id, acc, P,
+        metro_dispatch<T, false>(form.regs, grid, st, g, L, mu, p, mfac, e, sq, nhits, k0, k1, sweep, stream_id, acc, P,
                                  (float)beta);
 }
 template void launch_metropolis<double>(const Geom &, const LinkField<double> &, int, int, double, double, int,

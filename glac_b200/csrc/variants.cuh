@@ -15,6 +15,9 @@ constexpr int kMaxVariants = 4;
 struct VariantForm {
     int regs, shape;
 };
+inline bool operator==(const VariantForm &a, const VariantForm &b) { return a.regs == b.regs && a.shape == b.shape; }
+// several warps to a link (split.cu, metro_split.cu)
+constexpr VariantForm kSplitForm{-1, 0};
 
 // The flow stage waits on its neighbour links (L2 hits), so resident warps count
 // for more than registers: its caps give 16 (FP64) and 24 (FP32) warps per SM.
@@ -43,6 +46,28 @@ inline VariantForm variant_form(Family f, bool fp32, int v) {
 inline int metro_default_regs(bool fp32, bool learned, int blocks) {
     if (fp32) return learned || blocks <= 5 * 148 ? 128 : 96;
     return blocks > 10 * 148 ? 128 : 0;
+}
+
+// What a variant launches on a single lattice; split: whether its default is kSplitForm.
+// The other exponentials have one form, whose stage 1 with the measurement may still be
+// the site-per-thread one.
+inline VariantForm lattice_flow_form(bool fp32, int v, bool split, bool morningstar) {
+    if (v == 0 && split) return kSplitForm;
+    const VariantForm f = variant_form(FAM_FLOW, fp32, v);
+    return morningstar ? f : VariantForm{0, f.shape == 3 ? 3 : 0};
+}
+inline VariantForm lattice_metro_form(bool fp32, int v, bool split, bool learned, int blocks) {
+    if (v == 0 && split) return kSplitForm;
+    return v == 0 ? VariantForm{metro_default_regs(fp32, learned, blocks), 0} : variant_form(FAM_METRO, fp32, v);
+}
+
+// same[v]: the first variant with v's form.
+template <typename Form> void first_alike(int n, Form form, int *same) {
+    for (int v = 0; v < n; v++) {
+        same[v] = v;
+        for (int w = 0; w < v && same[v] == v; w++)
+            if (form(w) == form(v)) same[v] = w;
+    }
 }
 
 }  // namespace glac

@@ -166,8 +166,9 @@ glac_status glac_flow_stage_times_measured(glac_ctx *ctx, int n_steps, double *s
 
 /* Launch-variant autotuner (no reference counterpart): times each launch
  * variant (register cap / resident blocks per SM) of the flow-stage,
- * Metropolis and observable kernels on this lattice, reps calls each, keeps the
- * fastest, and restores the field and random stream.  report (may be NULL)
+ * Metropolis and observable kernels on this lattice, about reps calls each in
+ * turn (variants that launch the same kernel here once), keeps the fastest, and
+ * restores the field and random stream.  report (may be NULL)
  * receives 3 x 4 seconds-per-call entries [family][variant], 0 where unused. */
 glac_status glac_autotune(glac_ctx *ctx, int reps, double *report);
 /* The chosen variant per family (flow, metropolis, observables), and a setter

@@ -107,6 +107,15 @@ def test_autotune_leaves_chains_alone(g, ens):
             assert rel(E.get_links(i), F.get_links(i)) < 1e-4
 
 
+def test_autotune_times_a_kernel_once(g, ens):
+    with ens.Ensemble(DIMS, BETAS, precision="fp32", seed=SEED) as E:
+        E.hot_start(8)
+        rep = E.autotune(2)
+    for fam, same in (("flow", [0, 0, 2, 3]), ("metropolis", [0, 0, 2, 3])):
+        assert all(x > 0 for x in rep[fam])
+        assert [rep[fam][v] for v in same] == rep[fam]
+
+
 def test_ensemble_errors(g, ens):
     with pytest.raises(g.GlacError):
         ens.Ensemble([(4, 4, 4, 5)], [6.0])

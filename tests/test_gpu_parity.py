@@ -185,6 +185,23 @@ def test_autotune_restores_state_and_keeps_results(g, oracle):
                 assert_obs_close(A.flow(2), B.flow(2), TOL[prec], f"variant {v}")
 
 
+@pytest.mark.parametrize("prec, alike", [("fp64", {"flow": [0, 0, 2, 3], "metropolis": [0, 1]}),
+                                         ("fp32", {"flow": [0, 0, 2, 3], "metropolis": [0, 1, 2, 0]})])
+def test_autotune_times_a_kernel_once(g, prec, alike):
+    # 16^3 x 32 (512 blocks a sub-sweep): two numbers of one kernel get one time, and
+    # the fastest is chosen
+    with lattice(g, (16, 16, 16, 32), prec, seed=9) as L:
+        L.hot_start(2)
+        rep = L.autotune(3)
+        for fam, same in alike.items():
+            t = rep[fam][:len(same)]
+            assert all(x > 0 for x in t)
+            assert [t[v] for v in same] == t
+        for k, fam in enumerate(("flow", "metropolis", "observables")):
+            t = [x for x in rep[fam] if x > 0]
+            assert t[rep["chosen"][k]] == min(t)
+
+
 @pytest.mark.parametrize("prec", ["fp64", "fp32"])
 def test_flow_variants_agree(g, oracle, prec):
     # (z, t) pairs of two 128-site chunks and Nz, Nt multiples of 4, so the

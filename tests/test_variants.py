@@ -15,8 +15,8 @@ def lines(tmp_path_factory):
     subprocess.run(["g++", "-std=c++17", "-O1", "-I", os.path.join(ROOT, "glac_b200", "csrc"),
                     os.path.join(ROOT, "tests", "native", "variants.cpp"), "-o", exe], check=True)
 
-    def run(*blocks):
-        out = subprocess.run([exe, *map(str, blocks)], check=True, capture_output=True, text=True).stdout
+    def run(*args):
+        out = subprocess.run([exe, *map(str, args)], check=True, capture_output=True, text=True).stdout
         return [tuple(int(x) for x in line.split()) for line in out.splitlines()]
 
     return run
@@ -33,3 +33,15 @@ def test_numbers_keep_their_meaning(lines):
     for (f, p), per in want.items():
         for v, form in per.items():
             assert forms[f, p, v] == form, (f, p, v)
+
+
+@pytest.mark.parametrize("case, flow64, flow32, metro64, metro32", [
+    # split, Morningstar, learned, blocks of a sub-sweep
+    ((1, 1, 0, 32), (0, 1, 2, 3), (0, 1, 2, 3), (0, 1), (0, 1, 2, 3)),          # several warps to a link
+    ((0, 1, 0, 5 * 148), (0, 0, 2, 3), (0, 0, 2, 3), (0, 1), (0, 1, 2, 0)),     # one wave: 128 registers
+    ((0, 1, 0, 5 * 148 + 1), (0, 0, 2, 3), (0, 0, 2, 3), (0, 1), (0, 0, 2, 3)),  # 96
+    ((0, 1, 1, 8192), (0, 0, 2, 3), (0, 0, 2, 3), (0, 0), (0, 1, 2, 0)),        # learned; FP64 beyond ten blocks per SM
+    ((0, 0, 0, 1480), (0, 0, 0, 0), (0, 0, 2, 0), (0, 1), (0, 0, 2, 3)),        # another exponential
+    ((0, 0, 0, 1481), (0, 0, 0, 0), (0, 0, 2, 0), (0, 0), (0, 0, 2, 3))])
+def test_variants_that_launch_the_same_kernel(lines, case, flow64, flow32, metro64, metro32):
+    assert lines(*case) == [(FLOW, 0, *flow64), (FLOW, 1, *flow32), (METRO, 0, *metro64), (METRO, 1, *metro32)]
