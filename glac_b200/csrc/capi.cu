@@ -150,7 +150,7 @@ void reunit(glac_ctx *c) {
 
 // How this context's flow steps run.
 struct FlowMode {
-    bool split;      // each link's staple terms over six warps (split.cu)
+    bool split;      // a link's three planes on three warps (split.cu)
     bool in_stage1;  // the measurement's combination inside stage 1, else a pass of its own
     int nb;          // its partial sums per half time slice
     size_t row;      // doubles of one measurement's partial sums

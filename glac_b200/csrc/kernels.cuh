@@ -100,8 +100,7 @@ void launch_flow_stage1_combine(const Geom &g, const LinkField<T> &in, const Lin
                                 const ForceField<T> &zf, int kind, double alpha, double beta,
                                 const CloverParts<T> &cp, const ObsPlan &plan, double *partial, bool site,
                                 cudaStream_t st);
-// A Morningstar flow stage with each link's six staple terms on six warps
-// (split.cu).  With meas, stage 0 also writes the clover parts and stage 1
+// A Morningstar flow stage with each link's three planes on three warps (split.cu).  With meas, stage 0 also writes the clover parts and stage 1
 // combines them (where flow_split_combines holds) into the partial sums of a
 // plan of 32-site blocks, nb = V / (64 Nt).
 bool flow_split_combines(const Geom &g);

@@ -7,10 +7,13 @@
 // chain_wait until that kernel has ended and its writes are visible.  A kernel
 // launched this way calls chain_wait before its first access to anything that
 // an earlier kernel writes.  Whatever is launched otherwise waits for the whole
-// chain.  Kernels release late, before their last arithmetic: released at their
-// start, the waiting blocks of the next kernel crowd onto the SMs that have room
-// and leave it unbalanced (Metropolis sweep of 12^3 x 24 in FP32: 177 us, against
-// 132 without chaining).
+// chain.  Flow stages, sub-sweeps and the measurement's parts release late, before
+// their last arithmetic: released at their start, the waiting blocks of the next
+// kernel crowd onto the SMs that have room and leave it unbalanced (Metropolis sweep
+// of 12^3 x 24 in FP32: 177 us, against 132 without chaining).  The trainer's two
+// kernels release at their start: their blocks all fit beside one another, and the
+// gradient's fetch its rows before they wait.  Combinations and final sums, which are
+// short, never release; their end does.
 #pragma once
 
 #include <cuda_runtime.h>
