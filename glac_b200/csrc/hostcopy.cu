@@ -18,6 +18,7 @@
 
 #include <sched.h>
 #include <sys/mman.h>
+#include <unistd.h>
 
 namespace glac {
 
@@ -39,6 +40,7 @@ std::mutex g_hold_mu;   // g_holders and the buffers' lifetime
 int g_holders = 0;
 std::mutex g_use_mu;    // one transfer at a time
 void *g_mapped = nullptr;  // the buffers' mapping
+pid_t g_owner = 0;         // the process that made it
 char *g_pinned = nullptr;  // the buffers: kThreads x kSlots pieces
 size_t g_plain = 0;     // bytes that went the plain way for want of the buffers
 
@@ -141,20 +143,24 @@ cudaError_t split_copy(char *dev, char *host, size_t bytes, int device, cudaStre
 }
 
 // The buffers: whole huge pages where the system gives them, which are quick to
-// pin; a forked child gets none of them.
+// pin.  A forked child gets none of them (their pages must not become copies of
+// what the driver has pinned) and leaves what may lie at their place alone.
 void unpin_buffers() {
-    if (g_pinned) cudaHostUnregister(g_pinned);
+    if (g_owner == getpid()) {
+        if (g_pinned) cudaHostUnregister(g_pinned);
+        if (g_mapped) munmap(g_mapped, kPinnedBytes + kHugePage);
+    }
     g_pinned = nullptr;
-    if (g_mapped) munmap(g_mapped, kPinnedBytes + kHugePage);
     g_mapped = nullptr;
 }
 void pin_buffers() {
     void *m = mmap(nullptr, kPinnedBytes + kHugePage, PROT_READ | PROT_WRITE, MAP_PRIVATE | MAP_ANONYMOUS, -1, 0);
     if (m == MAP_FAILED) return;
     g_mapped = m;
+    g_owner = getpid();
     char *p = reinterpret_cast<char *>(((uintptr_t)m + kHugePage - 1) / kHugePage * kHugePage);
+    madvise(m, kPinnedBytes + kHugePage, MADV_DONTFORK);
     madvise(p, kPinnedBytes, MADV_HUGEPAGE);
-    madvise(p, kPinnedBytes, MADV_DONTFORK);
     for (size_t i = 0; i < kPinnedBytes; i += kHugePage) reinterpret_cast<volatile char *>(p)[i] = 0;
     if (cudaHostRegister(p, kPinnedBytes, cudaHostRegisterPortable) == cudaSuccess) {
         g_pinned = p;

@@ -5,6 +5,8 @@
 //   fail             the third and every later thread of the copies that follow finds no memory
 //   hold | drop      a holder comes or goes; drop prints the bytes pinned after it
 //   pinned           prints the bytes pinned now and how often memory was pinned
+//   forked           a child puts memory of its own where the buffers were, drops its
+//                    holder and uses that memory; prints its exit status
 #include "hostcopy.cu"
 
 #include <cstdio>
@@ -12,6 +14,7 @@
 #include <new>
 #include <sched.h>
 #include <string>
+#include <sys/wait.h>
 #include <vector>
 
 static std::atomic<int> g_copies{0};
@@ -108,6 +111,19 @@ int main(int argc, char **argv) {
             glac::hostcopy_drop();
             printf("%zu\n", pinned());
         } else if (s == "pinned") printf("%zu %d\n", pinned(), g_pins);
+        else if (s == "forked") {
+            fflush(stdout);
+            const pid_t child = fork();
+            if (child == 0) {
+                void *p = mmap(glac::g_mapped, 4096, PROT_READ | PROT_WRITE, MAP_PRIVATE | MAP_ANONYMOUS | MAP_FIXED, -1, 0);
+                glac::hostcopy_drop();
+                *static_cast<volatile char *>(p) = 1;
+                _exit(pinned() > 0 ? 0 : 2);  // nor does the child unpin what is not its own
+            }
+            int status = -1;
+            waitpid(child, &status, 0);
+            printf("%d\n", status);
+        }
         else {
             const size_t n = (size_t)atoll(argv[++i]);
             const bool up = s == "up";

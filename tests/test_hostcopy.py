@@ -69,3 +69,7 @@ def test_few_cores_copy_plainly(fake, cores, least):
     else:
         out = fake(*make, "up", least - 1, "down", least - 1, "up", least, "down", least, cores=cores)
         assert out == [[400], [400], [1], [1], [least // MB], [least // MB]]
+
+
+def test_a_forked_child_leaves_the_buffers_alone(fake):
+    assert fake("hold", "up", 64 * MB, "forked", "up", 64 * MB, "drop") == [[64], [0], [64], [0]]
