@@ -26,7 +26,7 @@ namespace {
 
 constexpr size_t kPiece = (size_t)1 << 20;
 constexpr int kThreads = 8, kSlots = 2;
-constexpr size_t kLeastSplit = (size_t)12 << 20;  // see split_bytes
+constexpr size_t kLeastSplit = (size_t)10 << 20;  // see split_bytes
 constexpr size_t kPinnedBytes = kThreads * kSlots * kPiece, kHugePage = (size_t)2 << 20;
 // The buffers cost 1.8 ms, 3.6 the first time, to make and give back (16 MB of huge
 // pages; 10 ms by cudaHostAlloc).  A copy of 64 MB saves that by itself (up
@@ -50,16 +50,17 @@ int usable_cores() {
     if (sched_getaffinity(0, sizeof(set), &set) == 0) return CPU_COUNT(&set);
     return (int)std::thread::hardware_concurrency();
 }
-// The size from which a copy is split.  From three cores on 12 MB, below which
-// starting the threads costs what they save; on two, where they only share the
-// copying that one thread does, 128 MB; on one never.  Microseconds plain / split,
-// up and then down, on a B200 host: 16 cores 9 MB 471 / 473, 485 / 491, 16 MB 829 /
-// 670, 830 / 648; 3 cores 16 MB 809 / 753, 781 / 793, 24 MB 1246 / 1048, 1159 / 1081;
-// 2 cores 24 MB 1204 / 1343, 1159 / 1303, 96 MB 8304 / 5648, 4548 / 5224, 192 MB
+// The size from which a copy is split: 10 MB on four cores or more, below which
+// starting the threads costs what they save; 16 MB on three; on two, where they only
+// share the copying that one thread does, 128 MB; on one never.  Microseconds plain /
+// split, up and then down, on a B200 host: 16 cores 8 MB 415 / 419, 406 / 394, 10 MB
+// 517 / 475, 510 / 448, 16 MB 829 / 670, 830 / 648; 4 cores 8 MB 425 / 523, 425 / 419,
+// 12 MB 620 / 579, 625 / 518; 3 cores 10 MB 510 / 554, 507 / 540, 16 MB 809 / 753, 781 /
+// 793; 2 cores 24 MB 1204 / 1343, 1159 / 1303, 96 MB 8304 / 5648, 4548 / 5224, 192 MB
 // 16627 / 11339, 9132 / 9577; 1 core 192 MB 17053 / 16090, 9774 / 16528.
 size_t split_bytes() {
     const int cores = usable_cores();
-    return cores >= 3 ? kLeastSplit : cores == 2 ? (size_t)128 << 20 : SIZE_MAX;
+    return cores >= 4 ? kLeastSplit : cores == 3 ? (size_t)16 << 20 : cores == 2 ? (size_t)128 << 20 : SIZE_MAX;
 }
 
 bool pageable(const void *host) {

@@ -15,7 +15,7 @@ MB = 1 << 20
 def fake(tmp_path_factory):
     exe = str(tmp_path_factory.mktemp("native") / "hostcopy_fake")
     cuda = os.environ.get("CUDA_HOME", "/usr/local/cuda")
-    subprocess.run(["g++", "-std=c++17", "-O1", "-x", "c++", "-I", os.path.join(cuda, "include"), "-I",
+    subprocess.run(["g++", "-std=c++17", "-O3", "-x", "c++", "-I", os.path.join(cuda, "include"), "-I",
                     os.path.join(ROOT, "glac_b200", "csrc"),
                     os.path.join(ROOT, "tests", "native", "hostcopy_fake.cpp"), "-o", exe, "-lpthread"], check=True)
 
@@ -58,8 +58,8 @@ def test_buffers_come_after_enough_small_copies(fake):
     assert fake(*part, *part) == ([[1]] * 6 + [[0]]) * 2
 
 
-@pytest.mark.parametrize("cores, least", [(1, None), (2, 128 * MB), (3, 12 * MB), (16, 12 * MB), (-2, 128 * MB),
-                                          (-8, 12 * MB), (0, None)])
+@pytest.mark.parametrize("cores, least", [(1, None), (2, 128 * MB), (3, 16 * MB), (4, 10 * MB), (16, 10 * MB),
+                                          (-2, 128 * MB), (-8, 10 * MB), (0, None)])
 def test_few_cores_copy_plainly(fake, cores, least):
     # one transfer each just below the size from which copies are split and, where
     # they never are, of 400 MB; with the buffers there, a transfer per MB from it on
